@@ -23,6 +23,7 @@
 namespace sd {
 
 int build_grid(sphdem_grid_t* g, const float* pos, sphdem_ctl_t* ctl, cudaStream_t st);
+int build_fluid(sphdem_ctx_t* c, cudaStream_t st);
 int gather_fluid(const sphdem_ctx_t* c, cudaStream_t st);
 int gather_wall(const sphdem_ctx_t* c, float support, float h, cudaStream_t st);
 int gather_wall_rho(const sphdem_ctx_t* c, cudaStream_t st);
@@ -182,8 +183,8 @@ int coupled_onestep(sphdem_ctx_t* c, const sphdem_params_t* p, bool shep, cudaSt
     TRY(rec(f->join, f->side));
     // main, up to the fork of the porosity branch
     if (build) {
-        if (!fluid_fresh) TRY(build_grid(&c->grid_sph, c->sph.pos, c->ctl, st));
-        if (!density_fresh) TRY(gather_fluid(c, st));
+        if (!fluid_fresh) TRY(build_fluid(c, st));
+        else if (!density_fresh) TRY(gather_fluid(c, st));
     }
     TRY(run_dem_aux(c, st));
     if (shep) TRY(gather_wall_rho(c, st));
@@ -283,8 +284,7 @@ void drop_entry(GraphEntry& e) {
 
 int loop_body(sphdem_ctx_t* c, const sphdem_params_t* p, bool shep, int coupled, cudaStream_t st) {
     if (coupled) return coupled_onestep(c, p, shep, st, true);
-    TRY(build_grid(&c->grid_sph, c->sph.pos, c->ctl, st));
-    TRY(gather_fluid(c, st));
+    TRY(build_fluid(c, st));
     return sph_onestep(c, p, shep, true, st);
 }
 
@@ -634,8 +634,7 @@ int sphdem_grid_build(sphdem_ctx_t* c, int kind, const sphdem_params_t* p, sphde
             // kernel attributes of the tensor-core porosity pass, set here --
             // eagerly, before any graph captures a step that launches it
             if (c->work.pfb) TRY(porosity_setup());
-            TRY(build_grid(&c->grid_sph, c->sph.pos, c->ctl, st));
-            return gather_fluid(c, st);
+            return build_fluid(c, st);
         case 1:
             TRY(build_grid(&c->grid_bnd, c->bnd.pos, c->ctl, st));
             if (!p) {
@@ -750,8 +749,7 @@ int jump_body(sphdem_ctx_t* c, const sphdem_params_t* p, const sphdem_jump_t* j,
         return SPHDEM_ERR_CUDA;
     }
     TRY(run_corrmax(j->net.out, c->sph.n, c->dem.n, j->scale, (float)j->substeps * p->dt, j->dev + 1, st));
-    TRY(build_grid(&c->grid_sph, c->sph.pos, c->ctl, st));
-    TRY(gather_fluid(c, st));
+    TRY(build_fluid(c, st));
     // the judge's density is the full density pass of the next plain step
     // (pressures, sorted copies, neighbour records), so that step can skip it
     TRY(run_density(c, p->support, p->h, false, true, true, p->rho0, p->c0, p->gamma, st, p->block_sph, p->lanes_sph,
@@ -1047,7 +1045,7 @@ int sphdem_profile_step(sphdem_ctx_t* c, const sphdem_params_t* p, int step, int
     int rc = SPHDEM_OK;
     do {
         mark();
-        if ((rc = build_grid(&c->grid_sph, c->sph.pos, c->ctl, st)) || (rc = gather_fluid(c, st))) break;
+        if ((rc = build_fluid(c, st))) break;
         mark();
         if (coupled && (rc = build_grid(&c->grid_dem, c->dem.pos, c->ctl, st))) break;
         mark();
