@@ -1,10 +1,13 @@
 // sph.cu -- WCSPH neighbour loops on the sorted fluid / wall copies.
 //
-// One thread per subject (or, for small systems, one warp per subject: the
-// launch option lanes = 32), subjects taken in cell order (grid order), so the
-// threads of a warp query the same few cell columns and their float4
-// neighbour loads hit the same L1 lines.  Neighbour membership uses the exact
-// FP32 predicates of the reference; the physics sums use contracted FP32.
+// One thread per subject (LANES = 1) or, for systems that leave the GPU idle
+// then, 4 or 8 lanes per subject whose sums run in the order of the one thread
+// and give the same bits (walk.cuh); or one warp per subject with a sum order
+// of its own (LANES = 32: the launch option lanes_sph = 32).  Subjects are
+// taken in cell order (grid order), so the lanes of a warp query the same few
+// cell columns and their float4 neighbour loads hit the same L1 lines.
+// Neighbour membership uses the exact FP32 predicates of the reference; the
+// physics sums use contracted FP32.
 //
 //   k_density        Kernel_shepard_sph + Kernel_density_sph + Kernel_pres_sph
 //                    (kernel/KERNEL_rho.py:6-82, kernel/KERNEL_pres.py:6-23) in
@@ -30,49 +33,64 @@
 // member: a sixth of the bytes, but the force pass re-trims the ranges and
 // decodes the bits).
 #include "common.cuh"
+#include "walk.cuh"
 
 namespace sd {
 
 namespace {
 
-// Subject of this thread (LANES = 1) or of this warp (LANES = 32), and the
-// neighbour visitor: a thread walks every slot of the ball-trimmed ranges; a
-// warp takes the ranges together and its lanes stride through each one.  The
-// warp form has 32x the parallelism for small systems; its sums are reduced
-// across lanes at the end (a different, equally valid FP32 summation order).
+extern __shared__ __align__(16) unsigned char sph_smem[];
+
+// Subject of this thread and its lane among the subject's LANES.
 template <int LANES>
 __device__ __forceinline__ int subject_index(int& lane) {
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    lane = LANES == 1 ? 0 : (int)(threadIdx.x & 31);
-    return (int)(LANES == 1 ? t : t >> 5);
+    lane = (int)(threadIdx.x % LANES);
+    return (int)(t / LANES);
 }
 
+// body(ok, j, q, r) over the members (exact d2 < s2) of this lane's subject: a
+// thread that walks every slot of the ball-trimmed ranges (LANES = 1), a warp
+// whose lanes stride through each range together (LANES = 32; its sums are
+// reduced across lanes at the end, a different, equally valid FP32 summation
+// order), or walk.cuh's walk.
 template <int LANES, class F>
-__device__ __forceinline__ void visit_ball(const Geo& g, float px, float py, float pz, float rq, int inst, int lane,
-                                           F&& body) {
-    if (LANES == 1) {
-        for_each_range_ball(g, px, py, pz, rq, inst, [&](int s, int e) {
-            for (int j = s; j < e; ++j) body(j);
+__device__ __forceinline__ void visit_members(const Geo& g, const float4* __restrict__ posm, bool mine,
+                                              const float4& p, float rq, float s2, int inst, int lane, F&& body) {
+    auto one = [&](int j) {
+        const float4 q = posm[j];
+        const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
+        if (r.d2 < s2) body(true, j, q, r);
+    };
+    if constexpr (LANES == 1) {
+        for_each_range_ball(g, p.x, p.y, p.z, rq, inst, [&](int s, int e) {
+            for (int j = s; j < e; ++j) one(j);
+        });
+    } else if constexpr (LANES == 32) {
+        warp_ranges_ball(g, p.x, p.y, p.z, rq, inst, [&](int s, int e) {
+            for (int j = s + lane; j < e; j += 32) one(j);
         });
     } else {
-        warp_ranges_ball(g, px, py, pz, rq, inst, [&](int s, int e) {
-            for (int j = s + lane; j < e; j += 32) body(j);
-        });
+        WarpWalk<LANES>* walks = reinterpret_cast<WarpWalk<LANES>*>(sph_smem);
+        warp_walk<LANES>(g, posm, mine, p.x, p.y, p.z, rq, s2, inst, walks[threadIdx.x >> 5], body);
     }
+}
+
+// Adds a b of this lane (0 if !ok) to the subject's sum.
+template <int LANES>
+__device__ __forceinline__ float lanes_fma(float acc, float a, float b) {
+    return LANES == 1 || LANES == 32 ? fmaf(a, b, acc) : ordered_fma<LANES == 32 ? 1 : LANES>(acc, a, b);
 }
 
 template <int LANES>
 __device__ __forceinline__ float lanes_sum(float v) {
-    return LANES == 1 ? v : warp_sum(v);
+    return LANES == 32 ? warp_sum(v) : v;
 }
 
-// Thread-per-subject walk of the ball-trimmed ranges, candidate by candidate
-// (the lanes of a warp, consecutive particles of one or two cells, mostly test
-// the same candidate together, so its load is one broadcast), body(j, q, r)
-// for the members.  With rows, the walk mask is recorded: each range is taken
-// in segments that end where a 32-bit mask word ends, the segment's member
-// bits gathered in a register and stored with the word.  Returns the slots
-// walked.
+// Thread-per-subject walk of the ball-trimmed ranges that records the walk mask
+// in rows: body(j, q, r) for the members; each range is taken in segments that
+// end where a 32-bit mask word ends, the segment's member bits gathered in a
+// register and stored with the word.  Returns the slots walked.
 template <class Body>
 __device__ __forceinline__ int walk_record(const Geo& g, const float4* __restrict__ posm, const float4& p, float rq,
                                            int inst, float s2, int32_t* __restrict__ rows, size_t n, int k, int cap,
@@ -93,18 +111,16 @@ __device__ __forceinline__ int walk_record(const Geo& g, const float4* __restric
                     m |= bit;
                 }
             }
-            if (rows) {
-                word |= m;
-                if (sh + (j1 - j0) == 32) {
-                    if ((b >> 5) < cap) rows[(size_t)(b >> 5) * n + k] = (int32_t)word;
-                    word = 0u;
-                }
+            word |= m;
+            if (sh + (j1 - j0) == 32) {
+                if ((b >> 5) < cap) rows[(size_t)(b >> 5) * n + k] = (int32_t)word;
+                word = 0u;
             }
             j0 = j1;
         }
         pos += e - s;
     });
-    if (rows && (pos & 31) && (pos >> 5) < cap) rows[(size_t)(pos >> 5) * n + k] = (int32_t)word;
+    if ((pos & 31) && (pos >> 5) < cap) rows[(size_t)(pos >> 5) * n + k] = (int32_t)word;
     return pos;
 }
 
@@ -134,14 +150,14 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
     pdl_launch();
     int lane;
     const int k = subject_index<LANES>(lane);
-    if (k >= a.n) return;
-    const int o = a.gs.order[k];
-    const float4 p = a.f_posm[k];
-    const int inst = inst_of(a.gs, o);
+    const bool mine = k < a.n;
+    const size_t n = (size_t)a.n;
+    const int o = mine ? a.gs.order[k] : 0;
+    const float4 p = mine ? a.f_posm[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int inst = mine ? inst_of(a.gs, o) : 0;
     float rho_sum = 0.0f, flt_sum = 0.0f;
+    if ((LANES == 1 || LANES == 32) && !mine) return;
     if (LANES == 1 && a.nbr != nullptr && a.fmt == SPHDEM_NBR_MASKS) {
-        // the walks, recording their walk masks
-        const size_t n = (size_t)a.n;
         int32_t* rows = a.nbr;
         const int wf = walk_record(a.gs, a.f_posm, p, a.rq, inst, a.s2, rows, n, k, a.cap,
                                    [&](int j, const float4& q, const D2& r) {
@@ -160,46 +176,36 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
         rows[(size_t)(2 * a.cap) * n + k] = wf;
         rows[(size_t)(2 * a.cap + 1) * n + k] = wb;
     } else {
-        // the walks, recording the member slots when the step keeps them
-        const bool list = LANES == 1 && a.nbr != nullptr;
-        const size_t n = (size_t)a.n;
-        int cf = 0, cb = 0;
-        visit_ball<LANES>(a.gs, p.x, p.y, p.z, a.rq, inst, lane, [&](int j) {
-            const float4 q = a.f_posm[j];
-            const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
-            if (r.d2 < a.s2) {
-                const float w = kern_w(a.kern, fast_sqrt(r.d2));
-                if (RHO) rho_sum += q.w * w;
-                if (FLT) flt_sum += a.f_vprev[j] * w;
-                if (list) {
-                    if (cf < a.cap) a.nbr[(size_t)cf * n + k] = j;
-                    ++cf;
-                }
+        const bool list = LANES != 32 && a.nbr != nullptr;
+        const int shift = (threadIdx.x & 31) - lane;  // first lane of this subject
+        int found = 0;                                // members so far (recorded in rows, up to the capacity)
+        const float* __restrict__ vprev = a.f_vprev;
+        int32_t* rows = a.nbr;
+        auto member = [&](bool ok, int j, const float4& q, const D2& r) {
+            const float w = ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f;
+            if (list && LANES == 1) {
+                if (found < a.cap) rows[(size_t)found * n + k] = j;
+                ++found;
+            } else if (list) {
+                const unsigned of = (__ballot_sync(0xffffffffu, ok) >> shift) & ((1u << (LANES & 31)) - 1u);
+                const int row = found + __popc(of & ((1u << lane) - 1u));
+                if (ok && row < a.cap) rows[(size_t)row * n + k] = j;
+                found += __popc(of);
             }
-        });
-        if (a.gb.ncl > 0) {
-            visit_ball<LANES>(a.gb, p.x, p.y, p.z, a.rq, inst, lane, [&](int j) {
-                const float4 q = a.b_posm[j];
-                const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
-                if (r.d2 < a.s2) {
-                    const float w = kern_w(a.kern, fast_sqrt(r.d2));
-                    if (RHO) rho_sum += q.w * w;
-                    if (FLT) flt_sum += a.b_vprev[j] * w;
-                    if (list) {
-                        if (cb < a.cap) a.nbr[(size_t)(a.cap + cb) * n + k] = j;
-                        ++cb;
-                    }
-                }
-            });
-        }
-        if (list) {
-            a.nbr[(size_t)(2 * a.cap) * n + k] = cf;
-            a.nbr[(size_t)(2 * a.cap + 1) * n + k] = cb;
-        }
+            if (RHO) rho_sum = lanes_fma<LANES>(rho_sum, ok ? q.w : 0.0f, w);
+            if (FLT) flt_sum = lanes_fma<LANES>(flt_sum, ok ? vprev[j] : 0.0f, w);
+        };
+        visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane, member);
+        if (list && mine && lane == 0) a.nbr[(size_t)(2 * a.cap) * n + k] = found;
+        found = 0;
+        vprev = a.b_vprev;
+        rows += (size_t)a.cap * n;
+        if (a.gb.ncl > 0) visit_members<LANES>(a.gb, a.b_posm, mine, p, a.rq, a.s2, inst, lane, member);
+        if (list && mine && lane == 0) a.nbr[(size_t)(2 * a.cap + 1) * n + k] = found;
     }
     if (RHO) rho_sum = lanes_sum<LANES>(rho_sum);
     if (FLT) flt_sum = lanes_sum<LANES>(flt_sum);
-    if (lane != 0) return;
+    if (lane != 0 || !mine) return;
     if (FLT) a.flt[o] = flt_sum;
     if (RHO) {
         const float flt = FLT ? flt_sum : a.flt[o];
@@ -235,20 +241,20 @@ __global__ void __launch_bounds__(256) k_density_wall(WallArgs a) {
     pdl_launch();
     int lane;
     const int k = subject_index<LANES>(lane);
-    if (k >= a.n) return;
-    const int o = a.gb.order[k];
-    const float4 p = a.b_posm[k];
-    const int inst = inst_of(a.gb, o);
+    const bool mine = k < a.n;
+    if ((LANES == 1 || LANES == 32) && !mine) return;
+    const int o = mine ? a.gb.order[k] : 0;
+    const float4 p = mine ? a.b_posm[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int inst = mine ? inst_of(a.gb, o) : 0;
     float rho_sum = 0.0f;
-    if (a.gs.ncl > 0) {
-        visit_ball<LANES>(a.gs, p.x, p.y, p.z, a.rq, inst, lane, [&](int j) {
-            const float4 q = a.f_posm[j];
-            const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
-            if (r.d2 < a.s2) rho_sum += q.w * kern_w(a.kern, fast_sqrt(r.d2));
-        });
-    }
+    if (a.gs.ncl > 0)
+        visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane,
+                             [&](bool ok, int j, const float4& q, const D2& r) {
+                                 const float w = ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f;
+                                 rho_sum = lanes_fma<LANES>(rho_sum, ok ? q.w : 0.0f, w);
+                             });
     rho_sum = lanes_sum<LANES>(rho_sum);
-    if (lane != 0) return;
+    if (lane != 0 || !mine) return;
     const float rho = rho_sum + a.b_self[k];
     a.rho[o] = rho;
     if (PRES) {
@@ -279,55 +285,97 @@ struct ForceArgs {
     float two_mu, eps_h2, g;
 };
 
-// Pair term shared by the fluid and wall loops.  MODE bit 1: acceleration,
-// bit 2: negative pressure gradient.
+// Pair terms of the fluid and wall loops.  MODE bit 1: acceleration (fx, fy,
+// fz to be added), bit 2: negative pressure gradient (c, and grad_i W in gx,
+// gy, gz: the sum takes -c grad W).
+struct Pair {
+    float fx, fy, fz, c, gx, gy, gz;
+};
 template <int MODE>
-__device__ __forceinline__ void force_pair(const ForceArgs& a, const D2& r, const float4& vi, float pr_i,
-                                           float p_i, float irho_i, const float4& q, const float4& rpj,
-                                           const float4* __restrict__ velp, int j, float3& acc, float3& pgf) {
+__device__ __forceinline__ Pair force_pair(const ForceArgs& a, const D2& r, const float4& vi, float pr_i, float p_i,
+                                           float irho_i, const float4& q, const float4& rpj, const float4& vj) {
+    Pair f;
     const float rinv = rsqrtf(r.d2);
     const float dist = r.d2 * rinv;
     const float dwr = kern_dw(a.kern, dist) * rinv;  // (dW/dr) / r
-    const float gx = dwr * r.dx, gy = dwr * r.dy, gz = dwr * r.dz;  // grad_i W
+    f.gx = dwr * r.dx;
+    f.gy = dwr * r.dy;
+    f.gz = dwr * r.dz;
     if (MODE & 1) {
         const float sc = q.w * (pr_i + rpj.z);
-        const float4 vj = velp[j];
         const float visc =
-            __fdividef(a.two_mu * (r.dx * gx + r.dy * gy + r.dz * gz) * irho_i * rpj.w, r.d2 + a.eps_h2);
+            __fdividef(a.two_mu * (r.dx * f.gx + r.dy * f.gy + r.dz * f.gz) * irho_i * rpj.w, r.d2 + a.eps_h2);
         const float mv = q.w * visc;
-        acc.x += mv * (vi.x - vj.x) - sc * gx;
-        acc.y += mv * (vi.y - vj.y) - sc * gy;
-        acc.z += mv * (vi.z - vj.z) - sc * gz;
+        f.fx = mv * (vi.x - vj.x) - sc * f.gx;
+        f.fy = mv * (vi.y - vj.y) - sc * f.gy;
+        f.fz = mv * (vi.z - vj.z) - sc * f.gz;
     }
-    if (MODE & 2) {
-        const float c = q.w * rpj.w * (rpj.y - p_i);
-        pgf.x -= c * gx;
-        pgf.y -= c * gy;
-        pgf.z -= c * gz;
+    if (MODE & 2) f.c = q.w * rpj.w * (rpj.y - p_i);
+    return f;
+}
+
+// Adds this lane's pair (nothing if !ok) to the subject's sums.
+template <int LANES, int MODE>
+__device__ __forceinline__ void force_sum(bool ok, const Pair& f, float3& acc, float3& pgf) {
+    if constexpr (LANES == 1 || LANES == 32) {
+        if (!ok) return;
+        if (MODE & 1) acc = make_float3(acc.x + f.fx, acc.y + f.fy, acc.z + f.fz);
+        if (MODE & 2) pgf = make_float3(fmaf(-f.c, f.gx, pgf.x), fmaf(-f.c, f.gy, pgf.y), fmaf(-f.c, f.gz, pgf.z));
+    } else {
+#pragma unroll
+        for (int s = 0; s < LANES; ++s) {
+            auto of = [&](float v) { return __shfl_sync(0xffffffffu, ok ? v : 0.0f, s, LANES); };
+            if (MODE & 1) acc = make_float3(acc.x + of(f.fx), acc.y + of(f.fy), acc.z + of(f.fz));
+            if (MODE & 2) {
+                const float c = of(f.c);
+                pgf = make_float3(fmaf(-c, of(f.gx), pgf.x), fmaf(-c, of(f.gy), pgf.y), fmaf(-c, of(f.gz), pgf.z));
+            }
+        }
     }
 }
 
 // The c member slots rows[t * n + k] recorded for subject k, in walk order,
-// four per round: their slots, then their positions, are loaded together so
-// the gathers overlap (the loop is latency bound).
-template <int MODE>
+// kUnroll per lane and round: their slots, then their fields, are loaded
+// together so the gathers overlap (the loop is latency bound).  With LANES > 1
+// all lanes of the warp call it; the rounds are the warp's.
+template <int LANES, int MODE>
 __device__ __forceinline__ void force_slots(const ForceArgs& a, const float4* __restrict__ posm,
                                             const float4* __restrict__ rp, const float4* __restrict__ vel,
                                             const int32_t* __restrict__ rows, int c, const float4& p,
-                                            const float4& vi, const float4& rpi, int k, float3& acc, float3& pgf) {
+                                            const float4& vi, const float4& rpi, int k, int lane, float3& acc,
+                                            float3& pgf) {
+    constexpr int kUnroll = LANES == 1 ? 4 : 2;
     const size_t n = (size_t)a.n;
-    for (int t = 0; t < c; t += 4) {
-        int js[4];
-        float4 qs[4];
+    const int trips = LANES == 1 ? c : __reduce_max_sync(0xffffffffu, c);
+    for (int t = 0; t < trips; t += kUnroll * LANES) {
+        int js[kUnroll];
+        float4 qs[kUnroll], rs[kUnroll], vs[kUnroll];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) js[u] = t + u < c ? rows[(size_t)(t + u) * n + k] : rows[(size_t)t * n + k];
+        for (int u = 0; u < kUnroll; ++u) {
+            const int i = t + u * LANES + lane;
+            js[u] = i < c ? rows[(size_t)i * n + k] : 0;
+        }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) qs[u] = posm[js[u]];
+        for (int u = 0; u < kUnroll; ++u) qs[u] = posm[js[u]];
+        if (LANES > 1) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < kUnroll; ++u) {
+                rs[u] = rp[js[u]];
+                vs[u] = vel[js[u]];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
             const D2 r = d2_exact(p.x, p.y, p.z, qs[u].x, qs[u].y, qs[u].z);
-            if (t + u < c && r.d2 > kR2Min)
-                force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, qs[u], rp[js[u]], vel, js[u], acc, pgf);
+            const bool ok = t + u * LANES + lane < c && r.d2 > kR2Min;
+            if (LANES == 1) {
+                if (ok)
+                    force_sum<1, MODE>(true, force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, qs[u], rp[js[u]], vel[js[u]]),
+                                       acc, pgf);
+            } else {
+                force_sum<LANES, MODE>(ok, force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, qs[u], rs[u], vs[u]), acc,
+                                       pgf);
+            }
         }
     }
 }
@@ -399,7 +447,8 @@ __device__ __forceinline__ bool force_members(const ForceArgs& a, const Geo& g, 
         for (int u = 0; u < 4; ++u) {
             const D2 r = d2_exact(p.x, p.y, p.z, qv[u].x, qv[u].y, qv[u].z);
             if (js[u] >= 0 && r.d2 > kR2Min)
-                force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, qv[u], rp[js[u]], vel, js[u], acc, pgf);
+                force_sum<1, MODE>(true, force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, qv[u], rp[js[u]], vel[js[u]]),
+                                   acc, pgf);
         }
     }
     return true;
@@ -411,18 +460,20 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
     pdl_launch();
     int lane;
     const int k = subject_index<LANES>(lane);
-    if (k >= a.n) return;
-    const int o = a.gs.order[k];
-    const float4 p = a.f_posm[k];
-    const float4 vi = a.f_vel[k];
-    const float4 rpi = a.f_rp[k];
-    const int inst = inst_of(a.gs, o);
+    const bool mine = k < a.n;
+    if ((LANES == 1 || LANES == 32) && !mine) return;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int o = mine ? a.gs.order[k] : 0;
+    const float4 p = mine ? a.f_posm[k] : zero;
+    const float4 vi = mine ? a.f_vel[k] : zero;
+    const float4 rpi = mine ? a.f_rp[k] : zero;
+    const int inst = mine ? inst_of(a.gs, o) : 0;
+    const size_t n = (size_t)a.n;
     float3 acc = make_float3(0.f, 0.f, 0.f), pgf = make_float3(0.f, 0.f, 0.f);
-    bool walk = true;
+    bool walk = mine;
     if (LANES == 1 && a.nbr != nullptr && a.fmt == SPHDEM_NBR_MASKS) {
         // the members recorded by the density pass (all with d2 < s2), in walk order
-        extern __shared__ int32_t force_tab[];
-        const size_t n = (size_t)a.n;
+        int32_t* force_tab = reinterpret_cast<int32_t*>(sph_smem);
         const int wf = a.nbr[(size_t)(2 * a.cap) * n + k], wb = a.nbr[(size_t)(2 * a.cap + 1) * n + k];
         if (wf <= 32 * a.cap && wb <= 32 * a.cap) {
             float3 af = acc, pf = pgf;
@@ -437,31 +488,33 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
                 pgf = pf;
             }
         }
-    } else if (LANES == 1 && a.nbr != nullptr) {
+    } else if (LANES != 32 && a.nbr != nullptr) {
         // the member slots recorded by the density pass (all with d2 < s2), in walk order
-        const size_t n = (size_t)a.n;
-        const int cf = a.nbr[(size_t)(2 * a.cap) * n + k], cb = a.nbr[(size_t)(2 * a.cap + 1) * n + k];
-        if (cf <= a.cap && cb <= a.cap) {
-            walk = false;
-            force_slots<MODE>(a, a.f_posm, a.f_rp, a.f_vel, a.nbr, cf, p, vi, rpi, k, acc, pgf);
-            force_slots<MODE>(a, a.b_posm, a.b_rp, a.b_vel, a.nbr + (size_t)a.cap * n, cb, p, vi, rpi, k, acc, pgf);
+        const int cf = mine ? a.nbr[(size_t)(2 * a.cap) * n + k] : 0;
+        const int cb = mine ? a.nbr[(size_t)(2 * a.cap + 1) * n + k] : 0;
+        const bool listed = cf <= a.cap && cb <= a.cap;
+        if (listed) walk = false;
+        if (LANES != 1 || listed) {
+            constexpr int G = LANES == 32 ? 1 : LANES;
+            force_slots<G, MODE>(a, a.f_posm, a.f_rp, a.f_vel, a.nbr, listed ? cf : 0, p, vi, rpi, k, lane, acc, pgf);
+            force_slots<G, MODE>(a, a.b_posm, a.b_rp, a.b_vel, a.nbr + (size_t)a.cap * n, listed ? cb : 0, p, vi, rpi,
+                                 k, lane, acc, pgf);
         }
     }
-    if (walk) {
-        visit_ball<LANES>(a.gs, p.x, p.y, p.z, a.rq, inst, lane, [&](int j) {
-            const float4 q = a.f_posm[j];
-            const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
-            if (r.d2 > kR2Min && r.d2 < a.s2)
-                force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, q, a.f_rp[j], a.f_vel, j, acc, pgf);
-        });
-        if (a.gb.ncl > 0) {
-            visit_ball<LANES>(a.gb, p.x, p.y, p.z, a.rq, inst, lane, [&](int j) {
-                const float4 q = a.b_posm[j];
-                const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
-                if (r.d2 > kR2Min && r.d2 < a.s2)
-                    force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, q, a.b_rp[j], a.b_vel, j, acc, pgf);
-            });
-        }
+    // subjects without a record (none kept, or one that overflowed): the walk
+    auto visit = [&](const Geo& g, const float4* __restrict__ posm, const float4* __restrict__ rp,
+                     const float4* __restrict__ vel) {
+        auto member = [&](bool ok, int j, const float4& q, const D2& r) {
+            ok = ok && r.d2 > kR2Min;
+            Pair f = {};
+            if (ok) f = force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, q, rp[j], vel[j]);
+            force_sum<LANES, MODE>(ok, f, acc, pgf);
+        };
+        visit_members<LANES>(g, posm, walk, p, a.rq, a.s2, inst, lane, member);
+    };
+    if (LANES == 1 || LANES == 32 ? walk : __any_sync(0xffffffffu, walk)) {
+        visit(a.gs, a.f_posm, a.f_rp, a.f_vel);
+        if (a.gb.ncl > 0) visit(a.gb, a.b_posm, a.b_rp, a.b_vel);
     }
     if (MODE & 1) {
         acc.x = lanes_sum<LANES>(acc.x);
@@ -473,7 +526,7 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
         pgf.y = lanes_sum<LANES>(pgf.y);
         pgf.z = lanes_sum<LANES>(pgf.z);
     }
-    if (lane != 0) return;
+    if (lane != 0 || !mine) return;
     if (MODE & 1) st3(a.acc, o, make_float3(acc.x, acc.y, acc.z - a.g));
     if (MODE & 2) {
         if (a.pgf) st3(a.pgf, o, pgf);
@@ -505,6 +558,70 @@ static float tait_B(float rho0, float c0, float gamma) { return rho0 * c0 * c0 /
 // Threads per block of the neighbour loops: 64, 128 or 256 (default 128).
 static int launch_block(int b) { return (b == 64 || b == 256) ? b : 128; }
 
+// Largest systems that take several lanes per subject; beyond them one thread
+// per subject fills the GPU and executes fewer instructions.  Measured (us, one
+// thread | several lanes):
+//   density (8 lanes)  12.5k: 114 | 34, 47k: 130 | 75, 752k: 580 | 897;
+//                      recording nothing, 100k: 95 | 119
+//   walls (4 lanes)    48k: 37 | 16, 118k: 40 | 21, 2.2M: 83 | 172
+//   force (4 lanes)    from records, 12.5k: 66 | 24, 47k: 67 | 47, 752k: 331 | 530;
+//                      by walks, 100k: 162 | 129
+constexpr int kDensityLanesMax = 128 * 1024, kDensityLanesMaxUnrecorded = 64 * 1024;
+constexpr int kWallLanesMax = 256 * 1024;
+constexpr int kForceLanesMax = 128 * 1024;
+
+// Blocks and shared memory of a loop with LANES lanes per subject (the walks
+// need 6-8 KB per warp: at most 128 threads, 48 KB without an opt-in).
+template <int LANES>
+static void loop_shape(int n, int& block, int& blocks, size_t& smem) {
+    if (LANES != 1 && LANES != 32 && block > 128) block = 128;
+    blocks = blocks_for((long)n * LANES, block);
+    smem = LANES == 1 || LANES == 32 ? 0 : (size_t)(block / 32) * sizeof(WarpWalk<LANES == 32 ? 1 : LANES>);
+}
+
+template <int LANES>
+static void launch_density(const DensArgs& a, bool flt, bool rho, bool pres, int bs, cudaStream_t st) {
+    int nb;
+    size_t smem;
+    loop_shape<LANES>(a.n, bs, nb, smem);
+    if (flt && rho && pres)
+        launch_pdl(k_density<LANES, true, true, true>, nb, bs, smem, st, a);
+    else if (!flt && rho && pres)
+        launch_pdl(k_density<LANES, false, true, true>, nb, bs, smem, st, a);
+    else if (flt && !rho)
+        launch_pdl(k_density<LANES, true, false, false>, nb, bs, smem, st, a);
+    else if (!flt && rho && !pres)
+        launch_pdl(k_density<LANES, false, true, false>, nb, bs, smem, st, a);
+    else
+        launch_pdl(k_density<LANES, true, true, false>, nb, bs, smem, st, a);
+}
+
+template <int LANES>
+static void launch_wall(const WallArgs& a, bool pres, int bs, cudaStream_t st) {
+    int nb;
+    size_t smem;
+    loop_shape<LANES>(a.n, bs, nb, smem);
+    if (pres)
+        launch_pdl(k_density_wall<LANES, true>, nb, bs, smem, st, a);
+    else
+        launch_pdl(k_density_wall<LANES, false>, nb, bs, smem, st, a);
+}
+
+template <int LANES>
+static void launch_force(const ForceArgs& a, int mode, int bs, cudaStream_t st) {
+    int nb;
+    size_t smem;
+    loop_shape<LANES>(a.n, bs, nb, smem);
+    if (LANES == 1 && a.nbr && a.fmt == SPHDEM_NBR_MASKS)  // the range tables (32 KB at 256 threads)
+        smem = (size_t)2 * kForceRanges * bs * sizeof(int32_t);
+    if (mode == 3)
+        launch_pdl(k_force<LANES, 3>, nb, bs, smem, st, a);
+    else if (mode == 2)
+        launch_pdl(k_force<LANES, 2>, nb, bs, smem, st, a);
+    else
+        launch_pdl(k_force<LANES, 1>, nb, bs, smem, st, a);
+}
+
 int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool rho, bool pres, float rho0, float c0,
                 float gamma, cudaStream_t st, int block, int lanes, int nbr_cap, int nbr_format) {
     const int n = c->sph.n;
@@ -533,31 +650,12 @@ int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool rh
     a.B = tait_B(rho0, c0, gamma);
     a.gamma = gamma;
     const int bs = launch_block(block);
-    if (lanes == 32) {
-        const int nb = blocks_for((long)n * 32, bs);
-        if (flt && rho && pres)
-            launch_pdl(k_density<32, true, true, true>, nb, bs, 0, st, a);
-        else if (!flt && rho && pres)
-            launch_pdl(k_density<32, false, true, true>, nb, bs, 0, st, a);
-        else if (flt && !rho)
-            launch_pdl(k_density<32, true, false, false>, nb, bs, 0, st, a);
-        else if (!flt && rho && !pres)
-            launch_pdl(k_density<32, false, true, false>, nb, bs, 0, st, a);
-        else
-            launch_pdl(k_density<32, true, true, false>, nb, bs, 0, st, a);
-    } else {
-        const int nb = blocks_for(n, bs);
-        if (flt && rho && pres)
-            launch_pdl(k_density<1, true, true, true>, nb, bs, 0, st, a);
-        else if (!flt && rho && pres)
-            launch_pdl(k_density<1, false, true, true>, nb, bs, 0, st, a);
-        else if (flt && !rho)
-            launch_pdl(k_density<1, true, false, false>, nb, bs, 0, st, a);
-        else if (!flt && rho && !pres)
-            launch_pdl(k_density<1, false, true, false>, nb, bs, 0, st, a);
-        else
-            launch_pdl(k_density<1, true, true, false>, nb, bs, 0, st, a);
-    }
+    if (lanes == 32)
+        launch_density<32>(a, flt, rho, pres, bs, st);
+    else if ((a.nbr && a.fmt == SPHDEM_NBR_MASKS) || n > (a.nbr ? kDensityLanesMax : kDensityLanesMaxUnrecorded))
+        launch_density<1>(a, flt, rho, pres, bs, st);
+    else
+        launch_density<8>(a, flt, rho, pres, bs, st);
     return launch_status("density");
 }
 
@@ -583,18 +681,12 @@ int run_density_wall(const sphdem_ctx_t* c, float support, float h, bool pres, f
     a.B = tait_B(rho0, c0, gamma);
     a.gamma = gamma;
     const int bs = launch_block(block);
-    if (lanes == 32) {
-        const int nb = blocks_for((long)n * 32, bs);
-        if (pres)
-            launch_pdl(k_density_wall<32, true>, nb, bs, 0, st, a);
-        else
-            launch_pdl(k_density_wall<32, false>, nb, bs, 0, st, a);
-    } else {
-        if (pres)
-            launch_pdl(k_density_wall<1, true>, blocks_for(n, bs), bs, 0, st, a);
-        else
-            launch_pdl(k_density_wall<1, false>, blocks_for(n, bs), bs, 0, st, a);
-    }
+    if (lanes == 32)
+        launch_wall<32>(a, pres, bs, st);
+    else if (n > kWallLanesMax)
+        launch_wall<1>(a, pres, bs, st);
+    else
+        launch_wall<4>(a, pres, bs, st);
     return launch_status("density_wall");
 }
 
@@ -626,25 +718,12 @@ int run_force(const sphdem_ctx_t* c, float support, float h, float mu, float g, 
     a.eps_h2 = 0.01f * h * h;
     a.g = g;
     const int bs = launch_block(block);
-    if (lanes == 32) {
-        const int nb = blocks_for((long)n * 32, bs);
-        if (mode == 3)
-            launch_pdl(k_force<32, 3>, nb, bs, 0, st, a);
-        else if (mode == 2)
-            launch_pdl(k_force<32, 2>, nb, bs, 0, st, a);
-        else
-            launch_pdl(k_force<32, 1>, nb, bs, 0, st, a);
-    } else {
-        const int nb = blocks_for(n, bs);
-        const size_t smem =
-            a.nbr && a.fmt == SPHDEM_NBR_MASKS ? (size_t)2 * kForceRanges * bs * sizeof(int32_t) : 0;  // 32 KB at 256
-        if (mode == 3)
-            launch_pdl(k_force<1, 3>, nb, bs, smem, st, a);
-        else if (mode == 2)
-            launch_pdl(k_force<1, 2>, nb, bs, smem, st, a);
-        else
-            launch_pdl(k_force<1, 1>, nb, bs, smem, st, a);
-    }
+    if (lanes == 32)
+        launch_force<32>(a, mode, bs, st);
+    else if ((a.nbr && a.fmt == SPHDEM_NBR_MASKS) || n > kForceLanesMax)
+        launch_force<1>(a, mode, bs, st);
+    else
+        launch_force<4>(a, mode, bs, st);
     return launch_status("force");
 }
 
