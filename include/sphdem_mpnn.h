@@ -93,14 +93,16 @@ typedef struct sphdem_mpnn_net {
     uint16_t* h3;             /* [n_recv,128]                                 */
     float* out;               /* [n_recv,16] FP32                             */
     int32_t* status;          /* device word, OR of SPHDEM_FLAG_* bits        */
-    /* optional (inference): the node layers then run on the receivers and on
-     * the non-receiver nodes that send an edge of the current graph only --
-     * the others' latent rows are never read (NULL: every node) */
+    /* optional: the node layers, and in the backward pass their gradients,
+     * then run on the receivers and on the non-receiver nodes that send an
+     * edge of the current graph only -- the others' latent rows are never read
+     * and have no gradient (NULL: every node).  The backward pass uses the list
+     * that the forward pass before it made. */
     int32_t* active;          /* [n_nodes] scratch flags                      */
     int32_t* active_list;     /* [1 + n_nodes - n_recv]: count, then nodes    */
 } sphdem_mpnn_net_t;
 
-/* Backward workspace. */
+/* Backward workspace (the [.., 128] buffers 16-byte aligned, as those above). */
 typedef struct sphdem_mpnn_grad {
     const float* d_out;       /* [n_recv,16] dL/d out                         */
     float* g2;                /* [n_recv,128]                                 */

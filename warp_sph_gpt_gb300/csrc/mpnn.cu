@@ -2,7 +2,7 @@
 // radius graph of all particles, trained and evaluated by tensor-core
 // (tcgen05, BF16 operands, FP32 accumulation in tensor memory) kernels.
 //
-// Kernels (all persistent, 128 threads = 4 warps = the 128 TMEM lanes):
+// Kernels (persistent, 512 threads: four per TMEM lane):
 //   k_rows     node MLP layers: Y = X W^T (+ bias, SiLU), one 128-row tile per
 //              MMA group; the weight image is bulk-copied (TMA) into shared
 //              memory once per CTA.
@@ -15,10 +15,13 @@
 //              both layers, forms dF, scatters dh0, and accumulates dW2 and
 //              dW1 across all of the CTA's tiles in TMEM.
 //   k_wgrad    weight gradients of the node layers, reduction over rows in
-//              TMEM, per-CTA partials reduced in a fixed order.
+//              TMEM, per-CTA partials reduced in a fixed order; the training
+//              pass runs them, and the node layers, on the receivers and the
+//              nodes that send (29k of 80k rows for a dam break member).
 // Every wait on an MMA or a bulk copy is bounded; on timeout the CTA raises
 // SPHDEM_FLAG_TIMEOUT, waits once more (bounded), frees its tensor memory and
 // returns.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <stdio.h>
 
@@ -172,6 +175,8 @@ __global__ void k_pack(const float* __restrict__ theta, uint16_t* __restrict__ p
 // ---------------------------------------------------------------------------
 // add (optional, K = 128): rows r < n_add of the A operand are A[r] + add[r]
 // (the residual h + s * sum_j f_ij (.) h_j, formed while staging the tile).
+// a_out (optional): the staged operand rows are stored there too.
+// EPI_F32: z_out (optional) receives the output as well.
 // list (optional): the layer runs on rows 0 .. n_direct - 1 and on the list[0]
 // rows list[1 ..] (in any order: rows are independent); M bounds both.
 template <int K, int N, int EPI, bool IMG>
@@ -180,7 +185,7 @@ __global__ void __launch_bounds__(kRT * kT) k_rows(const uint16_t* __restrict__ 
                                              const float* __restrict__ bias, float* __restrict__ out_f32,
                                              uint16_t* __restrict__ out_bf, float* __restrict__ z_out,
                                              int32_t* status, const int* __restrict__ list, int n_direct,
-                                             int early) {
+                                             int early, uint16_t* __restrict__ a_out) {
     constexpr uint32_t kB = N * K * 2, kA = kT * K * 2;
     constexpr uint32_t kCols = N < 32 ? 32 : N;
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -244,6 +249,7 @@ __global__ void __launch_bounds__(kRT * kT) k_rows(const uint16_t* __restrict__ 
                                pack2(bf((uint16_t)v.w) + a1.z, bf((uint16_t)(v.w >> 16)) + a1.w));
             }
             *reinterpret_cast<uint4*>(sA + tile_off(rt, 8 * q, K)) = v;
+            if (a_out && row < M) reinterpret_cast<uint4*>(a_out + (size_t)row * K)[q] = v;
         }
         operands_ready();
         if (tid == 0) {
@@ -271,9 +277,15 @@ __global__ void __launch_bounds__(kRT * kT) k_rows(const uint16_t* __restrict__ 
                 if (EPI == EPI_F32) {
                     float4* o = reinterpret_cast<float4*>(out_f32 + (size_t)row * N + c0);
 #pragma unroll
-                    for (int i = 0; i < W / 4; ++i)
-                        o[i] = make_float4(v[4 * i] + sbias[c0 + 4 * i], v[4 * i + 1] + sbias[c0 + 4 * i + 1],
-                                           v[4 * i + 2] + sbias[c0 + 4 * i + 2], v[4 * i + 3] + sbias[c0 + 4 * i + 3]);
+                    for (int i = 0; i < W; ++i) v[i] += sbias[c0 + i];
+#pragma unroll
+                    for (int i = 0; i < W / 4; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    if (z_out) {
+                        float4* o2 = reinterpret_cast<float4*>(z_out + (size_t)row * N + c0);
+#pragma unroll
+                        for (int i = 0; i < W / 4; ++i)
+                            o2[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    }
                 } else {
 #pragma unroll
                     for (int i = 0; i < W; ++i) v[i] += sbias[c0 + i];
@@ -311,8 +323,6 @@ struct EdgeArgs {
     float inv_r, inv_vs, inv_norm;
     const uint16_t* img_e1;
     const uint16_t* img_e2;
-    const uint16_t* img_e2t;
-    const float* b1;
     const float* b2;
     // forward: agg[r] += s * sum f (.) h[j]
     const uint16_t* h;
@@ -330,25 +340,6 @@ struct EdgeArgs {
     int32_t* status;
     int early;             // inference: the weight images are copied before the previous kernel is done
 };
-
-// Edge features of edge e (zeros past the end): ((x_j-x_i)/R, |x_j-x_i|/R,
-// (v_j-v_i)/v_s, 0...), as 16 BF16 values in two 16-byte words.
-__device__ __forceinline__ void edge_features(const EdgeArgs& a, int e, int E, int& r, int& j, uint4& q0) {
-    r = -1;
-    j = -1;
-    q0 = make_uint4(0, 0, 0, 0);
-    if (e >= E) return;
-    r = __ldg(a.receiver + e);
-    j = __ldg(a.sender + e);
-    const float4 pr = __ldg(a.pos + r), pj = __ldg(a.pos + j);
-    const float4 vr = __ldg(a.vel + r), vj = __ldg(a.vel + j);
-    const float dx = pj.x - pr.x, dy = pj.y - pr.y, dz = pj.z - pr.z;
-    const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
-    q0.x = pack2(dx * a.inv_r, dy * a.inv_r);
-    q0.y = pack2(dz * a.inv_r, dist * a.inv_r);
-    q0.z = pack2((vj.x - vr.x) * a.inv_vs, (vj.y - vr.y) * a.inv_vs);
-    q0.w = pack2((vj.z - vr.z) * a.inv_vs, 1.0f);
-}
 
 constexpr uint32_t kImg16 = 128 * 16 * 2;   // 4 KB
 constexpr uint32_t kImg128 = 128 * 128 * 2;  // 32 KB
@@ -389,6 +380,8 @@ __device__ __forceinline__ void edge_load_state(const EdgeArgs& a, EdgeLoad& L) 
     }
 }
 
+// Edge features: ((x_j-x_i)/R, |x_j-x_i|/R, (v_j-v_i)/v_s, 1) as 8 BF16 values
+// (zeros past the end); the other 8 input columns are zero.
 __device__ __forceinline__ uint4 edge_pack(const EdgeArgs& a, const EdgeLoad& L) {
     if (L.r < 0) return make_uint4(0, 0, 0, 0);
     const float dx = L.pj.x - L.pr.x, dy = L.pj.y - L.pr.y, dz = L.pj.z - L.pr.z;
@@ -639,213 +632,213 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
     }
 }
 
-// k_edges_bwd shared memory
-constexpr uint32_t EB_IMG1 = 0, EB_IMG2 = EB_IMG1 + kImg16, EB_IMG2T = EB_IMG2 + kImg128, EB_XS = EB_IMG2T + kImg128,
-                   EB_XT = EB_XS + kImg16, EB_ZR = EB_XT + kImg16, EB_ZT = EB_ZR + kImg128, EB_DFT = EB_ZT + kImg128,
-                   EB_DF = EB_DFT + kImg128, EB_B1 = EB_DF + kImg128, EB_B2 = EB_B1 + 512, EB_SR = EB_B2 + 512,
-                   EB_SJ = EB_SR + 512, EB_BARS = EB_SJ + 512, EB_SLOT = EB_BARS + 16, EB_BYTES = EB_SLOT + 16;
-static_assert(EB_BYTES <= 227 * 1024, "k_edges_bwd shared memory");
+// k_edges_bwd shared memory.  Every operand is stored once, by the rows its
+// epilogue owns, and enters its second product MN-major (umma.cuh): the hidden
+// tile Z by edges, dF by features, dP by hidden units (over Z's space), the
+// edge inputs by edges, W2 as the forward image.
+constexpr uint32_t EB_IMG1 = 0, EB_IMG2 = EB_IMG1 + kImg16, EB_XS = EB_IMG2 + kImg128, EB_ZR = EB_XS + kImg16,
+                   EB_DFT = EB_ZR + kImg128, EB_B2 = EB_DFT + kImg128, EB_SR = EB_B2 + 512, EB_SJ = EB_SR + 512,
+                   EB_MASK = EB_SJ + 512, EB_BARS = EB_MASK + 2048, EB_SLOT = EB_BARS + 16, EB_BYTES = EB_SLOT + 16;
+static_assert(2 * (EB_BYTES + 1024) <= 228 * 1024, "k_edges_bwd: two CTAs per SM");
+constexpr int kBT = 512;  // threads: warps w, w + 4, w + 8, w + 12 share 32 TMEM lanes and split the 128 columns
 
-// TMEM columns: [0,128) layer 1 then dZ; [128,256) layer 2; [256,384) dW2; [384,400) dW1.
-__global__ void __launch_bounds__(kT, 1) k_edges_bwd(EdgeArgs a) {
+// Backward of the first message round and of the edge MLP, per 128-edge tile:
+// layer 1 and layer 2 again, dF = g1 h0 + g2 h2, the scatter of dh0, dW2 +=
+// dF^T Z, dZ = W2^T dF^T, dP = dZ relu', dW1 += dP^T X.  What bounds it is the
+// work between the MMAs (per edge and feature: the products, a 4-byte atomic
+// add, two roundings), so it takes 4 threads per TMEM lane and two CTAs per SM
+// that fill each other's waits.  One thread per lane, one CTA per SM and
+// transposed copies of Z, dF and X written element by element took 1,108 us
+// for 509k edges; this form takes 254 us.
+// TMEM columns: [0,128) layer 1, layer 2, dZ, then dW1 of the tile; [128,256) dW2.
+__global__ void __launch_bounds__(kBT, 2) k_edges_bwd(EdgeArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
     uint8_t* img1 = sm + EB_IMG1;
     uint8_t* img2 = sm + EB_IMG2;
-    uint8_t* img2t = sm + EB_IMG2T;
     uint8_t* xs = sm + EB_XS;
-    uint8_t* xt = sm + EB_XT;
-    uint8_t* zr = sm + EB_ZR;  // Z rows (layer-2 B operand), then dP^T (dW1 A operand)
-    uint8_t* zt = sm + EB_ZT;
+    uint8_t* zr = sm + EB_ZR;  // Z rows, then dP rows
     uint8_t* dft = sm + EB_DFT;
-    uint8_t* dfr = sm + EB_DF;
-    float* b1 = reinterpret_cast<float*>(sm + EB_B1);
     float* b2 = reinterpret_cast<float*>(sm + EB_B2);
     int* sr = reinterpret_cast<int*>(sm + EB_SR);
     int* sj = reinterpret_cast<int*>(sm + EB_SJ);
+    uint32_t* mask = reinterpret_cast<uint32_t*>(sm + EB_MASK);  // [hidden unit / 32][edge]: z > 0
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + EB_BARS);
     uint32_t* slot = reinterpret_cast<uint32_t*>(sm + EB_SLOT);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lanes = 32 * (warp & 3), c0 = 32 * (warp >> 2);
+    const int row = lanes + (tid & 31);  // TMEM lane: edge, feature or hidden unit
     const int E = min(__ldg(a.offset + a.n_recv), a.cap);
 
-    const uint32_t tmem = cta_begin(bars, slot, 512);
-    b1[tid] = a.b1[tid];
-    b2[tid] = a.b2[tid];
+    const uint32_t tmem = cta_begin(bars, slot, 256);
+    if (tid < 128) b2[tid] = a.b2[tid];
     if (tid == 0) {
-        mbar_arrive_expect_tx(&bars[1], kImg16 + 2 * kImg128);
+        mbar_arrive_expect_tx(&bars[1], kImg16 + kImg128);
         tma_load_1d(img1, a.img_e1, kImg16, &bars[1]);
         tma_load_1d(img2, a.img_e2, kImg128, &bars[1]);
-        tma_load_1d(img2t, a.img_e2t, kImg128, &bars[1]);
     }
     bool failed = __syncthreads_or(!mbar_wait(&bars[1], 0, kPolls));
     bool mine = true, pending = false, first = true;
     uint32_t phase = 0;
     constexpr uint32_t id128 = umma::idesc_bf16(128, 128), id16 = umma::idesc_bf16(128, 16);
-    float db1 = 0.0f, db2 = 0.0f;
-    const int c = tid;
+    float db1 = 0.0f, db2 = 0.0f, w1[4] = {0.f, 0.f, 0.f, 0.f};
+    EdgeLoad nxt;
+    nxt.r = nxt.j = -1;
+    if (tid < kT) {
+        edge_load_ids(a, blockIdx.x * kT + tid, E, nxt);
+        edge_load_state(a, nxt);
+    }
     for (int tile = blockIdx.x; !failed && tile * kT < E; tile += gridDim.x) {
-        if (pending) {  // dW1 of the previous tile still reads xt and the dP^T tile
-            if (!mma_done(bars, phase, mine)) { failed = true; break; }
-            pending = false;
-        }
-        int r, j;
-        uint4 q0;
-        edge_features(a, tile * kT + tid, E, r, j, q0);
-        sr[tid] = r;
-        sj[tid] = j;
-        *reinterpret_cast<uint4*>(xs + tile_off(tid, 0, 16)) = q0;
-        *reinterpret_cast<uint4*>(xs + tile_off(tid, 8, 16)) = make_uint4(0, 0, 0, 0);
-        {
-            const uint32_t w[4] = {q0.x, q0.y, q0.z, q0.w};
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const uint16_t hv = i < kBiasCol ? (uint16_t)(w[i >> 1] >> (16 * (i & 1))) : (uint16_t)0;
-                *reinterpret_cast<uint16_t*>(xt + tile_off(i, tid, 128)) = hv;
-            }
+        if (tid < kT) {
+            sr[tid] = nxt.r;
+            sj[tid] = nxt.j;
+            *reinterpret_cast<uint4*>(xs + tile_off(tid, 0, 16)) = edge_pack(a, nxt);
+            *reinterpret_cast<uint4*>(xs + tile_off(tid, 8, 16)) = make_uint4(0, 0, 0, 0);
         }
         operands_ready();
         if (tid == 0) {
             umma::fence_after();
-            umma::mma_tile(tmem, xs, img1, 16, id128, false);
+            umma::mma_tile(tmem, xs, img1, 16, id128, false);  // P[e][k]
             umma::commit(&bars[0]);
         }
+        if (tid < kT) edge_load_ids(a, (tile + gridDim.x) * kT + tid, E, nxt);
         pending = true;
         if (!mma_done(bars, phase, mine)) { failed = true; break; }
         pending = false;
-        // layer-1 epilogue (row = edge): Z rows and Z^T
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
+        {  // lane = edge: Z row, z > 0
             float v[32];
-            umma::tmem_ld32(umma::taddr(tmem, 32 * warp, c0), v);
+            umma::tmem_ld32(umma::taddr(tmem, lanes, c0), v);
+            uint32_t on = 0u;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.0f);
+            for (int i = 0; i < 32; ++i) on |= v[i] > 0.0f ? 1u << i : 0u;
+            mask[(c0 >> 5) * kT + row] = on;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                *reinterpret_cast<uint4*>(zr + tile_off(tid, c0 + 8 * q, 128)) =
-                    make_uint4(pack2(v[8 * q], v[8 * q + 1]), pack2(v[8 * q + 2], v[8 * q + 3]),
-                               pack2(v[8 * q + 4], v[8 * q + 5]), pack2(v[8 * q + 6], v[8 * q + 7]));
-#pragma unroll
-            for (int i = 0; i < 32; ++i) st_bf16(zt, tile_off(c0 + i, tid, 128), v[i]);
+                *reinterpret_cast<uint4*>(zr + tile_off(row, c0 + 8 * q, 128)) =
+                    make_uint4(pack2_relu(v[8 * q], v[8 * q + 1]), pack2_relu(v[8 * q + 2], v[8 * q + 3]),
+                               pack2_relu(v[8 * q + 4], v[8 * q + 5]), pack2_relu(v[8 * q + 6], v[8 * q + 7]));
         }
         operands_ready();
         if (tid == 0) {
             umma::fence_after();
-            umma::mma_tile(tmem + 128, img2, zr, 128, id128, false);
+            umma::mma_tile(tmem, img2, zr, 128, id128, false);  // F[c][e]
             umma::commit(&bars[0]);
         }
+        if (tid < kT) edge_load_state(a, nxt);
         pending = true;
         if (!mma_done(bars, phase, mine)) { failed = true; break; }
         pending = false;
-        // layer-2 epilogue (lane = feature c): dF, scatter of dh0, db2
-        {
-            const float bc = b2[c];
+        {  // lane = feature: dF row, scatter of dh0, db2
+            const float bc = b2[row];
+            float v[32];
+            umma::tmem_ld32(umma::taddr(tmem, lanes, c0), v);
             int cur = -1;
             float g1v = 0.0f, g2v = 0.0f;
-#pragma unroll 1
-            for (int c0 = 0; c0 < 128; c0 += 32) {
-                float v[32], df[32];
-                umma::tmem_ld32(umma::taddr(tmem + 128, 32 * warp, c0), v);
-#pragma unroll 4
-                for (int i = 0; i < 32; ++i) {
-                    const int rr = sr[c0 + i], jj = sj[c0 + i];
-                    df[i] = 0.0f;
-                    if (rr < 0) continue;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const int rr = sr[c0 + i], jj = sj[c0 + i];
+                float df = 0.0f;
+                if (rr >= 0) {
                     if (rr != cur) {
                         cur = rr;
-                        g1v = __ldg(a.g1 + (size_t)rr * kH + c) * a.inv_norm;
-                        g2v = __ldg(a.g2 + (size_t)rr * kH + c) * a.inv_norm;
+                        g1v = __ldg(a.g1 + (size_t)rr * kH + row) * a.inv_norm;
+                        g2v = __ldg(a.g2 + (size_t)rr * kH + row) * a.inv_norm;
                     }
-                    const float h0v = bf(__ldg(a.h0 + (size_t)jj * kH + c));
-                    const float h2v = bf(__ldg(a.h2 + (size_t)jj * kH + c));
-                    df[i] = g1v * h0v + g2v * h2v;
-                    atomicAdd(a.dh0 + (size_t)jj * kH + c, (v[i] + bc) * g1v);
+                    const float h0v = bf(__ldg(a.h0 + (size_t)jj * kH + row));
+                    const float h2v = bf(__ldg(a.h2 + (size_t)jj * kH + row));
+                    df = g1v * h0v + g2v * h2v;
+                    atomicAdd(a.dh0 + (size_t)jj * kH + row, (v[i] + bc) * g1v);
                 }
-#pragma unroll
-                for (int i = 0; i < 32; ++i) db2 += df[i];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    *reinterpret_cast<uint4*>(dft + tile_off(c, c0 + 8 * q, 128)) =
-                        make_uint4(pack2(df[8 * q], df[8 * q + 1]), pack2(df[8 * q + 2], df[8 * q + 3]),
-                                   pack2(df[8 * q + 4], df[8 * q + 5]), pack2(df[8 * q + 6], df[8 * q + 7]));
-#pragma unroll
-                for (int i = 0; i < 32; ++i) st_bf16(dfr, tile_off(c0 + i, c, 128), df[i]);
+                db2 += df;
+                v[i] = df;
             }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(dft + tile_off(row, c0 + 8 * q, 128)) =
+                    make_uint4(pack2(v[8 * q], v[8 * q + 1]), pack2(v[8 * q + 2], v[8 * q + 3]),
+                               pack2(v[8 * q + 4], v[8 * q + 5]), pack2(v[8 * q + 6], v[8 * q + 7]));
         }
         operands_ready();
         if (tid == 0) {
             umma::fence_after();
-            umma::mma_tile(tmem + 256, dft, zt, 128, id128, !first);  // dW2[c][k] += dF^T Z
-            umma::mma_tile(tmem, img2t, dfr, 128, id128, false);      // dZ[k][e] = W2^T dF^T
+            umma::mma_tile_mn(tmem + 128, dft, 0, zr, 128, 128, id128 | umma::kBMn, !first);  // dW2[c][k] += dF^T Z
+            umma::mma_tile_mn(tmem, img2, 128, dft, 128, 128, id128 | umma::kAMn | umma::kBMn, false);  // dZ[k][e]
             umma::commit(&bars[0]);
         }
         pending = true;
         if (!mma_done(bars, phase, mine)) { failed = true; break; }
         pending = false;
-        // dZ epilogue (lane = hidden unit k): dP = dZ * relu'(P), db1, dP^T tile
-        {
-            const int k = tid;
-#pragma unroll 1
-            for (int c0 = 0; c0 < 128; c0 += 32) {
-                float v[32];
-                umma::tmem_ld32(umma::taddr(tmem, 32 * warp, c0), v);
+        {  // lane = hidden unit: dP row, db1
+            float v[32];
+            umma::tmem_ld32(umma::taddr(tmem, lanes, c0), v);
+            const uint4* on = reinterpret_cast<const uint4*>(mask + (warp & 3) * kT + c0);
+            const uint32_t bit = 1u << (tid & 31);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const uint4 zq = *reinterpret_cast<const uint4*>(zt + tile_off(k, c0 + 8 * q, 128));
-                    const uint32_t zw[4] = {zq.x, zq.y, zq.z, zq.w};
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const uint16_t zb = (uint16_t)(zw[i >> 1] >> (16 * (i & 1)));
-                        if (!(bf(zb) > 0.0f)) v[8 * q + i] = 0.0f;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 32; ++i) db1 += v[i];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    *reinterpret_cast<uint4*>(zr + tile_off(k, c0 + 8 * q, 128)) =
-                        make_uint4(pack2(v[8 * q], v[8 * q + 1]), pack2(v[8 * q + 2], v[8 * q + 3]),
-                                   pack2(v[8 * q + 4], v[8 * q + 5]), pack2(v[8 * q + 6], v[8 * q + 7]));
+            for (int q = 0; q < 8; ++q) {
+                const uint4 m = on[q];
+                if (!(m.x & bit)) v[4 * q] = 0.0f;
+                if (!(m.y & bit)) v[4 * q + 1] = 0.0f;
+                if (!(m.z & bit)) v[4 * q + 2] = 0.0f;
+                if (!(m.w & bit)) v[4 * q + 3] = 0.0f;
             }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) db1 += v[i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(zr + tile_off(row, c0 + 8 * q, 128)) =
+                    make_uint4(pack2(v[8 * q], v[8 * q + 1]), pack2(v[8 * q + 2], v[8 * q + 3]),
+                               pack2(v[8 * q + 4], v[8 * q + 5]), pack2(v[8 * q + 6], v[8 * q + 7]));
         }
         operands_ready();
         if (tid == 0) {
             umma::fence_after();
-            umma::mma_tile(tmem + 384, zr, xt, 128, id16, !first);  // dW1[k][in] += dP^T X
+            umma::mma_tile_mn(tmem, zr, 0, xs, 16, 128, id16 | umma::kBMn, false);  // dW1[k][in] of this tile
             umma::commit(&bars[0]);
         }
         pending = true;
+        if (!mma_done(bars, phase, mine)) { failed = true; break; }
+        pending = false;
+        {
+            float v[4];
+            umma::tmem_ld4(umma::taddr(tmem, lanes, c0 >> 3), v);  // this thread's 4 of the 16 inputs
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w1[i] += v[i];
+        }
         first = false;
     }
-    if (!failed && pending) {
-        failed = !mma_done(bars, phase, mine);
-        if (!failed) pending = false;
-    }
     float* part = a.partial + (size_t)blockIdx.x * kBwdStride;
+    __syncthreads();
     if (!failed) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
-            float v[32];
-            umma::tmem_ld32(umma::taddr(tmem + 256, 32 * warp, c0), v);
+        float v[32];
+        umma::tmem_ld32(umma::taddr(tmem + 128, lanes, c0), v);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) part[tid * 128 + c0 + i] = first ? 0.0f : v[i];
-        }
-        {
-            float v[16];
-            umma::tmem_ld16(umma::taddr(tmem + 384, 32 * warp, 0), v);
+        for (int i = 0; i < 32; ++i) part[row * 128 + c0 + i] = first ? 0.0f : v[i];
+        const int in = c0 >> 3;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) part[128 * 128 + tid * 16 + i] = first ? 0.0f : v[i];
+        for (int i = 0; i < 4; ++i) part[128 * 128 + row * 16 + in + i] = in + i < kBiasCol ? w1[i] : 0.0f;
+        float* red = reinterpret_cast<float*>(dft);  // the four threads of a lane, in order
+        red[tid] = db1;
+        red[kBT + tid] = db2;
+        __syncthreads();
+        if (warp < 4) {
+            part[128 * 128 + 128 * 16 + tid] = ((red[tid] + red[tid + 128]) + red[tid + 256]) + red[tid + 384];
+            const float* r2 = red + kBT;
+            part[128 * 128 + 128 * 16 + 128 + tid] = ((r2[tid] + r2[tid + 128]) + r2[tid + 256]) + r2[tid + 384];
         }
-        part[128 * 128 + 128 * 16 + tid] = db1;
-        part[128 * 128 + 128 * 16 + 128 + tid] = db2;
     }
-    cta_end(bars, phase, pending && !mine, tmem, 512, a.status, failed);
+    cta_end(bars, phase, pending && !mine, tmem, 256, a.status, failed);
 }
 
 // ---------------------------------------------------------------------------
 // weight gradients of the node layers: C[128][N] = sum_r P[r][:]^T Q[r][:]
 // ---------------------------------------------------------------------------
+// Both operands are staged by rows (16-byte stores, 8 rows x 64 bytes per
+// warp) and enter the product MN-major; 512 threads stage and read out.  With
+// list, the rows are 0 .. n_direct - 1 and the list[0] rows list[1 ..], as in
+// k_rows; n_rows bounds both.  80k rows: 53 us with one thread per row and
+// transposed 2-byte stores; 27 us for the 29k rows that take part.
 template <int N>
-__global__ void __launch_bounds__(kT) k_wgrad(const uint16_t* __restrict__ P, const uint16_t* __restrict__ Q, int rows,
-                                              float* __restrict__ partial, int32_t* status) {
+__global__ void __launch_bounds__(kRT * kT) k_wgrad(const uint16_t* __restrict__ P, const uint16_t* __restrict__ Q,
+                                                    int n_rows, const int* __restrict__ list, int n_direct,
+                                                    float* __restrict__ partial, int32_t* status) {
     constexpr uint32_t kA = 128 * 128 * 2, kB = N * 128 * 2;
     constexpr uint32_t kCols = N < 32 ? 32 : N;
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -853,37 +846,33 @@ __global__ void __launch_bounds__(kT) k_wgrad(const uint16_t* __restrict__ P, co
     uint8_t* sB = sm + kA;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sB + kB);
     uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lanes = 32 * (warp & 3), grp = warp >> 2;
     const uint32_t tmem = cta_begin(bars, slot, kCols);
     bool mine = true, failed = false, pending = false, first = true;
     uint32_t phase = 0;
-    constexpr uint32_t idesc = umma::idesc_bf16(128, N);
+    constexpr uint32_t idesc = umma::idesc_bf16(128, N) | umma::kAMn | umma::kBMn;
+    const int rows = list ? min(n_rows, n_direct + __ldg(list)) : n_rows;
+    auto stage = [&](uint8_t* to, const uint16_t* from, int chunk, int cols) {
+        // (rows / 8) x (cols / 32) warp pieces of 8 rows x 4 16-byte words
+        const int per = max(cols / 32, 1), words = cols / 8;
+        for (int w = warp; w < 16 * per; w += kRT * 4) {
+            const int r = 8 * (w / per) + (lane & 7), q = 4 * (w % per) + (lane >> 3);
+            if (q >= words) continue;
+            int row = chunk * kT + r;
+            if (list && row >= n_direct) row = row < rows ? __ldg(list + 1 + (row - n_direct)) : n_rows;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (row < n_rows && chunk * kT + r < rows)
+                v = __ldg(reinterpret_cast<const uint4*>(from + (size_t)row * cols) + q);
+            *reinterpret_cast<uint4*>(to + tile_off(r, 8 * q, cols)) = v;
+        }
+    };
     for (int chunk = blockIdx.x; chunk * kT < rows; chunk += gridDim.x) {
-        const int row = chunk * kT + tid;
-#pragma unroll 1
-        for (int q = 0; q < 16; ++q) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (row < rows) v = __ldg(reinterpret_cast<const uint4*>(P + (size_t)row * 128) + q);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                *reinterpret_cast<uint16_t*>(sA + tile_off(8 * q + i, tid, 128)) =
-                    (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
-        }
-#pragma unroll 1
-        for (int q = 0; q < N / 8; ++q) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (row < rows) v = __ldg(reinterpret_cast<const uint4*>(Q + (size_t)row * N) + q);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                *reinterpret_cast<uint16_t*>(sB + tile_off(8 * q + i, tid, 128)) =
-                    (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
-        }
+        stage(sA, P, chunk, 128);
+        stage(sB, Q, chunk, N);
         operands_ready();
         if (tid == 0) {
             umma::fence_after();
-            umma::mma_tile(tmem, sA, sB, 128, idesc, !first);
+            umma::mma_tile_mn(tmem, sA, 128, sB, N, 128, idesc, !first);
             umma::commit(&bars[0]);
         }
         pending = true;
@@ -892,95 +881,135 @@ __global__ void __launch_bounds__(kT) k_wgrad(const uint16_t* __restrict__ P, co
         first = false;
     }
     if (!failed) {
-        float* part = partial + (size_t)blockIdx.x * 128 * N;
+        float* part = partial + (size_t)blockIdx.x * 128 * N + (lanes + lane) * N;
+        if (N < 32) {
+            float v[4];
+            umma::tmem_ld4(umma::taddr(tmem, lanes, 4 * grp), v);
 #pragma unroll
-        for (int c0 = 0; c0 < N; c0 += (N < 32 ? 16 : 32)) {
+            for (int i = 0; i < 4; ++i) part[4 * grp + i] = first ? 0.0f : v[i];
+        } else {
             float v[32];
-            if (N < 32)
-                umma::tmem_ld16(umma::taddr(tmem, 32 * warp, c0), v);
-            else
-                umma::tmem_ld32(umma::taddr(tmem, 32 * warp, c0), v);
+            umma::tmem_ld32(umma::taddr(tmem, lanes, 32 * grp), v);
 #pragma unroll
-            for (int i = 0; i < (N < 32 ? 16 : 32); ++i) part[tid * N + c0 + i] = first ? 0.0f : v[i];
+            for (int i = 0; i < 32; ++i) part[32 * grp + i] = first ? 0.0f : v[i];
         }
     }
     cta_end(bars, phase, pending && !mine, tmem, kCols, status, failed);
 }
 
-// dst[i] (or dst transposed) = sum over ctas of partial[cta * stride + off + i], fixed order.
-__global__ void k_reduce(const float* __restrict__ partial, int ncta, int stride, int off, int count, int rows_t,
-                         int cols_t, float* __restrict__ dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float s = 0.0f;
-    for (int b = 0; b < ncta; ++b) s += partial[(size_t)b * stride + off + i];
-    if (rows_t > 0) {  // source [rows_t][cols_t] -> destination [cols_t][rows_t]
-        const int a = i / cols_t, b = i % cols_t;
-        dst[b * rows_t + a] = s;
-    } else {
-        dst[i] = s;
+// Sums of per-CTA partials, in a fixed order: segment s is `count` sums over n
+// partials of `stride` floats at src, written to dst (transposed from
+// [rows_t][cols_t] when rows_t > 0).  A CTA takes 32 sums; its 8 warps each add
+// every eighth partial (a thread that adds all of them waits for one load
+// after another: 15 us per segment; all ten segments take 12 us now).
+struct Segment {
+    const float* src;
+    float* dst;
+    int n, stride, count, rows_t, cols_t;
+};
+constexpr int kSegments = 10;
+struct Segments {
+    Segment s[kSegments];
+    int n;
+};
+__global__ void __launch_bounds__(256) k_reduce(Segments g) {
+    __shared__ float red[8][32];
+    int b = blockIdx.x, k = 0;
+    while (k < g.n && b >= (g.s[k].count + 31) / 32) b -= (g.s[k++].count + 31) / 32;
+    if (k >= g.n) return;
+    const Segment s = g.s[k];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = 32 * b + lane;
+    float t = 0.0f;
+    if (i < s.count) {
+#pragma unroll 8
+        for (int p = w; p < s.n; p += 8) t += s.src[(size_t)p * s.stride + i];
     }
-}
-
-// Column sums of a row-major [rows][cols] FP32 matrix, deterministic.
-__global__ void k_colsum_part(const float* __restrict__ m, int rows, int cols, int chunk, float* __restrict__ part) {
-    const int c = threadIdx.x;
-    if (c >= cols) return;
-    const int r0 = blockIdx.x * chunk, r1 = min(rows, r0 + chunk);
-    float s = 0.0f;
-    for (int r = r0; r < r1; ++r) s += m[(size_t)r * cols + c];
-    part[blockIdx.x * cols + c] = s;
+    red[w][lane] = t;
+    __syncthreads();
+    if (w != 0 || i >= s.count) return;
+#pragma unroll
+    for (int p = 1; p < 8; ++p) t += red[p][lane];
+    s.dst[s.rows_t > 0 ? (i % s.cols_t) * s.rows_t + i / s.cols_t : i] = t;
 }
 
 // ---------------------------------------------------------------------------
 // elementwise pieces
 // ---------------------------------------------------------------------------
-// out[r] = h[r] + agg[r] for r < n_recv, h[r] otherwise (BF16 rows of 128).
-__global__ void k_residual(const uint16_t* __restrict__ h, const float* __restrict__ agg, int n_recv, int rows,
-                           uint16_t* __restrict__ out) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;  // pair index
-    if (i >= (long)rows * 64) return;
-    const long r = i / 64;
-    const uint32_t hw = reinterpret_cast<const uint32_t*>(h)[i];
-    float a = bf((uint16_t)hw), b = bf((uint16_t)(hw >> 16));
-    if (r < n_recv) {
-        const float2 g = reinterpret_cast<const float2*>(agg)[i];
-        a += g.x;
-        b += g.y;
+// Row of index i in the node order of k_rows: 0 .. n_direct - 1, then the list.
+__device__ __forceinline__ int node_row(int i, int n_direct, const int* __restrict__ list) {
+    return list && i >= n_direct ? __ldg(list + 1 + (i - n_direct)) : i;
+}
+
+// Sum over the 8 row groups of a CTA of 256 threads (32 threads x 4 columns
+// each), written to part[blockIdx.x * cols ..].
+__device__ __forceinline__ void store_colsum(float4 s, int cols, float* __restrict__ part) {
+    __shared__ float4 red[8][32];
+    const int t = threadIdx.x & 31, g = threadIdx.x >> 5;
+    red[g][t] = s;
+    __syncthreads();
+    if (g != 0 || 4 * t >= cols) return;
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+        const float4 o = red[k][t];
+        s = make_float4(s.x + o.x, s.y + o.y, s.z + o.z, s.w + o.w);
     }
-    reinterpret_cast<uint32_t*>(out)[i] = pack2(a, b);
+    reinterpret_cast<float4*>(part + (size_t)blockIdx.x * cols)[t] = s;
 }
 
-// d <- d * silu'(z) (in place), BF16 copy.
-__global__ void k_act_grad(float* __restrict__ d, const float* __restrict__ z, long n, uint16_t* __restrict__ out) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = d[i] * silu_grad(z[i]);
-    d[i] = v;
-    out[i] = bf16_bits(v);
+// out = d * silu'(z) as BF16 and its column sums (one partial row per CTA), for
+// the node rows of the layer.
+__global__ void __launch_bounds__(256) k_act_grad(const float* __restrict__ d, const float* __restrict__ z, int n_rows,
+                                                  const int* __restrict__ list, int n_direct,
+                                                  uint16_t* __restrict__ out, float* __restrict__ part) {
+    const int rows = list ? min(n_rows, n_direct + __ldg(list)) : n_rows;
+    const int t = threadIdx.x & 31;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < rows; i += gridDim.x * 8) {
+        const size_t at = (size_t)node_row(i, n_direct, list) * kH / 4 + t;
+        const float4 dv = reinterpret_cast<const float4*>(d)[at], zv = reinterpret_cast<const float4*>(z)[at];
+        const float4 v = make_float4(dv.x * silu_grad(zv.x), dv.y * silu_grad(zv.y), dv.z * silu_grad(zv.z),
+                                     dv.w * silu_grad(zv.w));
+        reinterpret_cast<uint2*>(out)[at] = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+        s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+    }
+    store_colsum(s, kH, part);
 }
 
-__global__ void k_to_bf16(const float* __restrict__ s, long n, uint16_t* __restrict__ out) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = bf16_bits(s[i]);
+// The output gradient [n][16]: BF16 copy and column sums; zeroes the gradient
+// rows dh of the nodes that only send (the scatter adds to them).
+__global__ void __launch_bounds__(256) k_out_grad(const float* __restrict__ d, int n, uint16_t* __restrict__ out,
+                                                  float* __restrict__ part, float* __restrict__ dh, int n_nodes,
+                                                  const int* __restrict__ list) {
+    const int t = threadIdx.x & 31, g = threadIdx.x >> 5;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < 4)
+        for (int i = blockIdx.x * 8 + g; i < n; i += gridDim.x * 8) {
+            const float* q = d + (size_t)i * 16 + 4 * t;  // the caller's: any alignment
+            const float4 v = make_float4(q[0], q[1], q[2], q[3]);
+            reinterpret_cast<uint2*>(out)[(size_t)i * 4 + t] = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+            s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+        }
+    const int rows = list ? min(n_nodes, n + __ldg(list)) : n_nodes;
+    for (int i = n + blockIdx.x * 8 + g; i < rows; i += gridDim.x * 8)
+        reinterpret_cast<float4*>(dh)[(size_t)node_row(i, n, list) * kH / 4 + t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    store_colsum(s, 16, part);
 }
 
-// d_h2 = g2 on receiver rows, 0 elsewhere.
-__global__ void k_init_rows(const float* __restrict__ g, int n_recv, int rows, float* __restrict__ d) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)rows * kH) return;
-    d[i] = i < (long)n_recv * kH ? g[i] : 0.0f;
-}
-
-__global__ void __launch_bounds__(1024) k_loss(const float* __restrict__ out, const float* __restrict__ target, int n,
-                                               float* __restrict__ loss, float* __restrict__ d_out) {
+// Loss and its gradient: one cluster of 8 CTAs (16,759 rows: 9.6 us; one CTA
+// took 122), whose sums meet in the first CTA's shared memory in a fixed order.
+constexpr int kLossCtas = 8;
+__global__ void __cluster_dims__(kLossCtas, 1, 1) __launch_bounds__(1024)
+    k_loss(const float* __restrict__ out, const float* __restrict__ target, int n, float* __restrict__ loss,
+           float* __restrict__ d_out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
     __shared__ float red[32];
+    __shared__ float sums[kLossCtas];
     const float inv = n > 0 ? 1.0f / (6.0f * (float)n) : 0.0f;
     float s = 0.0f;
-    for (long i = threadIdx.x; i < (long)n * 16; i += blockDim.x) {
-        const int col = (int)(i & 15);
+    for (long i = blockIdx.x * 1024L + threadIdx.x; i < (long)n * 16; i += kLossCtas * 1024L) {
         float g = 0.0f;
-        if (col < 6) {
+        if ((i & 15) < 6) {
             const float d = out[i] - target[i];
             s += d * d;
             g = 2.0f * d * inv;
@@ -991,9 +1020,14 @@ __global__ void __launch_bounds__(1024) k_loss(const float* __restrict__ out, co
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x < 32) {
-        float t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) *loss = t * inv;
+        const float t = warp_sum(red[threadIdx.x]);
+        if (threadIdx.x == 0) cluster.map_shared_rank(sums, 0)[cluster.block_rank()] = t;
+    }
+    cluster.sync();
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+        float t = 0.0f;
+        for (int k = 0; k < kLossCtas; ++k) t += sums[k];
+        *loss = t * inv;
     }
 }
 
@@ -1226,7 +1260,7 @@ int smem_opt_in(Kern k, uint32_t bytes) {
 template <int K, int N, int EPI, bool IMG>
 int rows(const uint16_t* A, int M, const uint16_t* B, const float* bias, float* out_f32, uint16_t* out_bf,
          float* z_out, int32_t* status, cudaStream_t st, const float* add = nullptr, int n_add = 0,
-         const int* list = nullptr, int n_direct = 0, int early = 0) {
+         const int* list = nullptr, int n_direct = 0, int early = 0, uint16_t* a_out = nullptr) {
     if (M <= 0) return SPHDEM_OK;
     constexpr uint32_t bytes = N * K * 2 + kT * K * 2 + 4 * (N < 2 ? 2 : N) + 16 + 16;
     int rc = smem_opt_in(k_rows<K, N, EPI, IMG>, bytes);
@@ -1234,13 +1268,13 @@ int rows(const uint16_t* A, int M, const uint16_t* B, const float* bias, float* 
     const int tiles = (M + kT - 1) / kT;
     const int grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
     launch_pdl(k_rows<K, N, EPI, IMG>, grid, kRT * kT, bytes, st, A, M, add, n_add, B, bias, out_f32, out_bf, z_out, status,
-               list, n_direct, early);
+               list, n_direct, early, a_out);
     return launch_status("mpnn rows");
 }
 
 template <int N>
 int wgrad(const uint16_t* P, const uint16_t* Q, int n_rows, float* partial, int& ncta, int32_t* status,
-          cudaStream_t st) {
+          cudaStream_t st, const int* list = nullptr, int n_direct = 0) {
     constexpr uint32_t bytes = 128 * 128 * 2 + N * 128 * 2 + 16 + 16;
     int rc = smem_opt_in(k_wgrad<N>, bytes);
     if (rc) return rc;
@@ -1248,25 +1282,20 @@ int wgrad(const uint16_t* P, const uint16_t* Q, int n_rows, float* partial, int&
     ncta = chunks < 1 ? 1 : chunks;
     if (ncta > sm_count()) ncta = sm_count();
     if (ncta > kMaxCtas) ncta = kMaxCtas;
-    k_wgrad<N><<<ncta, kT, bytes, st>>>(P, Q, n_rows, partial, status);
+    k_wgrad<N><<<ncta, kRT * kT, bytes, st>>>(P, Q, n_rows, list, n_direct, partial, status);
     return launch_status("mpnn wgrad");
 }
 
-int reduce(const float* partial, int ncta, int stride, int off, int count, int rows_t, int cols_t, float* dst,
-           cudaStream_t st) {
-    k_reduce<<<blocks_for(count, 256), 256, 0, st>>>(partial, ncta, stride, off, count, rows_t, cols_t, dst);
-    return launch_status("mpnn reduce");
+void add_segment(Segments& g, const float* src, int n, int stride, int count, float* dst, int rows_t = 0,
+                 int cols_t = 0) {
+    g.s[g.n++] = {src, dst, n, stride, count, rows_t, cols_t};
 }
 
-int colsum(const float* m, int n_rows, int cols, float* part, float* dst, cudaStream_t st) {
-    int nb = 2 * sm_count();
-    int chunk = (n_rows + nb - 1) / nb;
-    if (chunk < 1) chunk = 1;
-    nb = (n_rows + chunk - 1) / chunk;
-    if (nb < 1) nb = 1;
-    k_colsum_part<<<nb, 128, 0, st>>>(m, n_rows, cols, chunk, part);
-    k_reduce<<<1, 128, 0, st>>>(part, nb, cols, 0, cols, 0, 0, dst);
-    return launch_status("mpnn colsum");
+int reduce(const Segments& g, cudaStream_t st) {
+    int blocks = 0;
+    for (int k = 0; k < g.n; ++k) blocks += (g.s[k].count + 31) / 32;
+    if (blocks > 0) k_reduce<<<blocks, 256, 0, st>>>(g);
+    return launch_status("mpnn reduce");
 }
 
 EdgeArgs edge_args(const sphdem_mpnn_net_t* n) {
@@ -1284,8 +1313,6 @@ EdgeArgs edge_args(const sphdem_mpnn_net_t* n) {
     a.inv_norm = n->inv_norm;
     a.img_e1 = n->packed + P_E1;
     a.img_e2 = n->packed + P_E2;
-    a.img_e2t = n->packed + P_E2T;
-    a.b1 = n->theta + SPHDEM_MPNN_E1_B;
     a.b2 = n->theta + SPHDEM_MPNN_E2_B;
     a.status = n->status;
     return a;
@@ -1398,9 +1425,10 @@ extern "C" int sphdem_mpnn_forward(const sphdem_mpnn_net_t* n, int store_pre, sp
     }
     cudaStream_t st = as_stream(stream);
     const int nn = n->n_nodes, nr = n->n_recv;
-    // inference: node layers on the receivers and the other nodes that send
+    // node layers on the receivers and the other nodes that send (no other
+    // node's rows are read, and none has a gradient)
     const int* list = nullptr;
-    if (!store_pre && n->active && n->active_list && nn > nr) {
+    if (n->active && n->active_list && nn > nr) {
         cudaError_t e = zero_words(n->active, nn, st);
         if (e == cudaSuccess) e = zero_words(n->active_list, 1, st);
         if (e != cudaSuccess) {
@@ -1413,7 +1441,7 @@ extern "C" int sphdem_mpnn_forward(const sphdem_mpnn_net_t* n, int store_pre, sp
     }
     int rc = rows<16, 128, EPI_SILU, true>(n->x, nn, n->packed + P_N1, n->theta + SPHDEM_MPNN_N1_B, nullptr, n->h0,
                                            store_pre ? n->z0 : nullptr, n->status, st, nullptr, 0, list, nr,
-                                           list != nullptr);
+                                           list != nullptr && !store_pre);
     if (rc) return rc;
     // Inference copies the weight images early: every kernel of the chain
     // runs behind kernels that do not write them (the first node layer only
@@ -1430,26 +1458,14 @@ extern "C" int sphdem_mpnn_forward(const sphdem_mpnn_net_t* n, int store_pre, sp
         a.h = round == 0 ? n->h0 : n->h2;
         a.agg = n->agg;
         if (nr > 0 && (rc = edges<MODE_AGG>(a, eg, st))) return rc;
-        if (round == 0) {
-            if (store_pre) {  // the backward pass needs h1 itself
-                k_residual<<<blocks_for((long)nn * 64, 256), 256, 0, st>>>(n->h0, n->agg, nr, nn, n->h1);
-                rc = rows<128, 128, EPI_SILU, true>(n->h1, nn, n->packed + P_N2, n->theta + SPHDEM_MPNN_N2_B,
-                                                    nullptr, n->h2, n->z2, n->status, st);
-            } else {  // h1 = h0 + agg formed while staging
-                rc = rows<128, 128, EPI_SILU, true>(n->h0, nn, n->packed + P_N2, n->theta + SPHDEM_MPNN_N2_B,
-                                                    nullptr, n->h2, nullptr, n->status, st, n->agg, nr, list, nr, 1);
-            }
-            if (rc) return rc;
-        } else if (store_pre) {
-            k_residual<<<blocks_for((long)nr * 64, 256), 256, 0, st>>>(n->h2, n->agg, nr, nr, n->h3);
-        }
+        if (round == 0)  // h1 = h0 + agg formed while staging (the backward pass reads it)
+            if ((rc = rows<128, 128, EPI_SILU, true>(n->h0, nn, n->packed + P_N2, n->theta + SPHDEM_MPNN_N2_B, nullptr,
+                                                     n->h2, store_pre ? n->z2 : nullptr, n->status, st, n->agg, nr,
+                                                     list, nr, !store_pre, store_pre ? n->h1 : nullptr)))
+                return rc;
     }
-    if (store_pre)
-        rc = rows<128, 16, EPI_F32, true>(n->h3, nr, n->packed + P_N3, n->theta + SPHDEM_MPNN_N3_B, n->out, nullptr,
-                                          nullptr, n->status, st);
-    else
-        rc = rows<128, 16, EPI_F32, true>(n->h2, nr, n->packed + P_N3, n->theta + SPHDEM_MPNN_N3_B, n->out, nullptr,
-                                          nullptr, n->status, st, n->agg, nr, nullptr, 0, 1);
+    rc = rows<128, 16, EPI_F32, true>(n->h2, nr, n->packed + P_N3, n->theta + SPHDEM_MPNN_N3_B, n->out, nullptr, nullptr,
+                                      n->status, st, n->agg, nr, nullptr, 0, !store_pre, store_pre ? n->h3 : nullptr);
     if (rc) return rc;
     return launch_status("mpnn_forward");
 }
@@ -1463,68 +1479,78 @@ extern "C" int sphdem_mpnn_backward(const sphdem_mpnn_net_t* n, const sphdem_mpn
     }
     cudaStream_t st = as_stream(stream);
     const int nn = n->n_nodes, nr = n->n_recv;
-    const long nh = (long)nn * kH;
+    // the node rows of the forward pass
+    const int* list = n->active && n->active_list && nn > nr ? n->active_list : nullptr;
     float* grad = g->grad;
     int ncta = 0, rc;
+    // every kernel below leaves per-CTA partials at a place of its own; one
+    // launch at the end sums them all
+    Segments sums;
+    sums.n = 0;
+    float* part = g->partial;
+    const float* const end = part + (size_t)kMaxCtas * kBwdStride;
+    const int bg = edge_grid(n, 2), cg = min(2 * sm_count(), kMaxCtas);
+    if (part + (size_t)bg * kBwdStride + (size_t)sm_count() * 128 * (16 + 128 + 16) + (size_t)cg * (16 + 128 + 128) > end) {
+        set_error_msg("mpnn_backward: partials larger than their buffer");
+        return SPHDEM_ERR_INVALID;
+    }
+    auto take = [&](int n_part, int stride) {
+        float* p = part;
+        part += (size_t)n_part * stride;
+        return p;
+    };
     // output layer
-    k_to_bf16<<<blocks_for((long)nr * 16, 256), 256, 0, st>>>(g->d_out, (long)nr * 16, g->bf_b);
-    if ((rc = wgrad<16>(n->h3, g->bf_b, nr, g->partial, ncta, n->status, st))) return rc;
-    if ((rc = reduce(g->partial, ncta, 128 * 16, 0, 128 * 16, 128, 16, grad + SPHDEM_MPNN_N3_W, st))) return rc;
-    if ((rc = colsum(g->d_out, nr, 16, g->partial, grad + SPHDEM_MPNN_N3_B, st))) return rc;
-    if ((rc = rows<16, 128, EPI_F32, true>(g->bf_b, nr, n->packed + P_N3T, nullptr, g->g2, nullptr, nullptr,
+    float* p = take(cg, 16);
+    k_out_grad<<<cg, 256, 0, st>>>(g->d_out, nr, g->bf_b, p, g->d_h2, nn, list);
+    add_segment(sums, p, cg, 16, 16, grad + SPHDEM_MPNN_N3_B);
+    if ((rc = wgrad<16>(n->h3, g->bf_b, nr, part, ncta, n->status, st))) return rc;
+    add_segment(sums, take(ncta, 128 * 16), ncta, 128 * 16, 128 * 16, grad + SPHDEM_MPNN_N3_W, 128, 16);
+    // second message round: d_h2 = g2 on the receivers, + the scatter
+    if ((rc = rows<16, 128, EPI_F32, true>(g->bf_b, nr, n->packed + P_N3T, nullptr, g->g2, nullptr, g->d_h2,
                                            n->status, st)))
         return rc;
-    // second message round
-    k_init_rows<<<blocks_for(nh, 256), 256, 0, st>>>(g->g2, nr, nn, g->d_h2);
     EdgeArgs a = edge_args(n);
     a.g = g->g2;
     a.dh = g->d_h2;
     if (nr > 0 && (rc = edges<MODE_SCATTER>(a, edge_grid(n, 1), st))) return rc;
     // second node layer
-    k_act_grad<<<blocks_for(nh, 256), 256, 0, st>>>(g->d_h2, n->z2, nh, g->bf_a);
-    if ((rc = wgrad<128>(g->bf_a, n->h1, nn, g->partial, ncta, n->status, st))) return rc;
-    if ((rc = reduce(g->partial, ncta, 128 * 128, 0, 128 * 128, 0, 0, grad + SPHDEM_MPNN_N2_W, st))) return rc;
-    if ((rc = colsum(g->d_h2, nn, 128, g->partial, grad + SPHDEM_MPNN_N2_B, st))) return rc;
-    if ((rc = rows<128, 128, EPI_F32, true>(g->bf_a, nn, n->packed + P_N2T, nullptr, g->d_h1, nullptr, nullptr,
-                                            n->status, st)))
+    p = take(cg, 128);
+    k_act_grad<<<cg, 256, 0, st>>>(g->d_h2, n->z2, nn, list, nr, g->bf_a, p);
+    add_segment(sums, p, cg, 128, 128, grad + SPHDEM_MPNN_N2_B);
+    if ((rc = wgrad<128>(g->bf_a, n->h1, nn, part, ncta, n->status, st, list, nr))) return rc;
+    add_segment(sums, take(ncta, 128 * 128), ncta, 128 * 128, 128 * 128, grad + SPHDEM_MPNN_N2_W);
+    // first message round and the edge MLP: d_h0 = d_h1, + the scatter
+    if ((rc = rows<128, 128, EPI_F32, true>(g->bf_a, nn, n->packed + P_N2T, nullptr, g->d_h1, nullptr, g->d_h0,
+                                            n->status, st, nullptr, 0, list, nr)))
         return rc;
-    // first message round and the edge MLP
-    cudaError_t e = cudaMemcpyAsync(g->d_h0, g->d_h1, sizeof(float) * (size_t)nh, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) {
-        set_error("mpnn_backward", e);
-        return SPHDEM_ERR_CUDA;
-    }
     a.g1 = g->d_h1;
     a.g2 = g->g2;
     a.h0 = n->h0;
     a.h2 = n->h2;
     a.dh0 = g->d_h0;
-    a.partial = g->partial;
-    const int bg = edge_grid(n, 1);
     if ((rc = smem_opt_in(k_edges_bwd, EB_BYTES))) return rc;
     if (nr > 0) {
-        k_edges_bwd<<<bg, kT, EB_BYTES, st>>>(a);
+        a.partial = take(bg, kBwdStride);
+        k_edges_bwd<<<bg, kBT, EB_BYTES, st>>>(a);
         if ((rc = launch_status("mpnn edges_bwd"))) return rc;
-        if ((rc = reduce(g->partial, bg, kBwdStride, 0, 128 * 128, 0, 0, grad + SPHDEM_MPNN_E2_W, st))) return rc;
-        if ((rc = reduce(g->partial, bg, kBwdStride, 128 * 128, 128 * 16, 0, 0, grad + SPHDEM_MPNN_E1_W, st)))
-            return rc;
-        if ((rc = reduce(g->partial, bg, kBwdStride, 128 * 128 + 128 * 16, 128, 0, 0, grad + SPHDEM_MPNN_E1_B, st)))
-            return rc;
-        if ((rc = reduce(g->partial, bg, kBwdStride, 128 * 128 + 128 * 16 + 128, 128, 0, 0, grad + SPHDEM_MPNN_E2_B,
-                         st)))
-            return rc;
+        add_segment(sums, a.partial, bg, kBwdStride, 128 * 128, grad + SPHDEM_MPNN_E2_W);
+        add_segment(sums, a.partial + 128 * 128, bg, kBwdStride, 128 * 16, grad + SPHDEM_MPNN_E1_W);
+        add_segment(sums, a.partial + 128 * 128 + 128 * 16, bg, kBwdStride, 128, grad + SPHDEM_MPNN_E1_B);
+        add_segment(sums, a.partial + 128 * 128 + 128 * 16 + 128, bg, kBwdStride, 128, grad + SPHDEM_MPNN_E2_B);
     } else {
-        e = cudaMemsetAsync(grad, 0, sizeof(float) * SPHDEM_MPNN_N1_W, st);
+        const cudaError_t e = cudaMemsetAsync(grad, 0, sizeof(float) * SPHDEM_MPNN_N1_W, st);
         if (e != cudaSuccess) {
             set_error("mpnn_backward", e);
             return SPHDEM_ERR_CUDA;
         }
     }
     // first node layer
-    k_act_grad<<<blocks_for(nh, 256), 256, 0, st>>>(g->d_h0, n->z0, nh, g->bf_a);
-    if ((rc = wgrad<16>(g->bf_a, n->x, nn, g->partial, ncta, n->status, st))) return rc;
-    if ((rc = reduce(g->partial, ncta, 128 * 16, 0, 128 * 16, 0, 0, grad + SPHDEM_MPNN_N1_W, st))) return rc;
-    if ((rc = colsum(g->d_h0, nn, 128, g->partial, grad + SPHDEM_MPNN_N1_B, st))) return rc;
+    p = take(cg, 128);
+    k_act_grad<<<cg, 256, 0, st>>>(g->d_h0, n->z0, nn, list, nr, g->bf_a, p);
+    add_segment(sums, p, cg, 128, 128, grad + SPHDEM_MPNN_N1_B);
+    if ((rc = wgrad<16>(g->bf_a, n->x, nn, part, ncta, n->status, st, list, nr))) return rc;
+    add_segment(sums, take(ncta, 128 * 16), ncta, 128 * 16, 128 * 16, grad + SPHDEM_MPNN_N1_W);
+    if ((rc = reduce(sums, st))) return rc;
     return launch_status("mpnn_backward");
 }
 
@@ -1534,7 +1560,7 @@ extern "C" int sphdem_mpnn_loss(const float* out, const float* target, int32_t n
         set_error_msg("mpnn_loss: invalid arguments");
         return SPHDEM_ERR_INVALID;
     }
-    k_loss<<<1, 1024, 0, as_stream(stream)>>>(out, target, n, loss, d_out);
+    k_loss<<<kLossCtas, 1024, 0, as_stream(stream)>>>(out, target, n, loss, d_out);
     return launch_status("mpnn_loss");
 }
 
@@ -1670,5 +1696,8 @@ extern "C" int sphdem_mpnn_wgrad(const uint16_t* p, const uint16_t* q, float* c,
     else
         rc = wgrad<128>(p, q, n_rows, partial, ncta, status, st);
     if (rc) return rc;
-    return reduce(partial, ncta, 128 * n, 0, 128 * n, 0, 0, c, st);
+    Segments sums;
+    sums.n = 0;
+    add_segment(sums, partial, ncta, 128 * n, 128 * n, c);
+    return reduce(sums, st);
 }

@@ -12,6 +12,12 @@
 // One MMA consumes K = 16 (two core matrices along K); the next K-slice
 // starts 256 B further.
 //
+// The same tile of R rows of C columns serves as the transposed operand (MN-
+// major: the columns are the operand's M or N, the rows its K): the core
+// matrices adjacent along the columns are 128 B apart (stride byte offset),
+// those of the next 8 rows C*16 B (leading byte offset), a K-slice of 16 rows
+// C*32 B.  So an operand is staged once, by rows, for both products it enters.
+//
 // D[M x N] (+)= A[M x K] * B[N x K]^T, M = 128 (one TMEM lane per row of D,
 // N FP32 columns), issued by one thread; completion is signalled on an
 // mbarrier by tcgen05.commit.  Thread t of warp w (w < 4) of the epilogue
@@ -45,6 +51,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, int K) {
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+
+// As smem_desc, for a tile of rows of C columns used MN-major.
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, int C) {
+    uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(((uint32_t)C * 16u) >> 4) << 16;
+    d |= (uint64_t)(128u >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    return d;
+}
+
+// idesc_bf16 with A (bit 15) or B (bit 16) MN-major.
+constexpr uint32_t kAMn = 1u << 15, kBMn = 1u << 16;
 
 // ---- tensor memory ---------------------------------------------------------
 // Warp-collective; the base address is written to *slot (shared memory).
@@ -90,6 +108,19 @@ __device__ __forceinline__ void mma_tile(uint32_t tmem_d, const void* a, const v
                  (accumulate || k > 0) ? 1u : 0u);
 }
 
+// D (+)= A * B^T over K, where an operand with C columns > 0 (ca, cb) is a tile of
+// K rows of C columns used MN-major (idesc has its bit), and one with C = 0 is
+// K-major as in mma_tile.  Single thread.
+__device__ __forceinline__ void mma_tile_mn(uint32_t tmem_d, const void* a, int ca, const void* b, int cb, int K,
+                                            uint32_t idesc, bool accumulate) {
+    const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+    for (int k = 0; k < K / 16; ++k) {
+        const uint64_t da = ca ? smem_desc_mn(sa + 32u * (uint32_t)ca * k, ca) : smem_desc(sa + 256u * k, K);
+        const uint64_t db = cb ? smem_desc_mn(sb + 32u * (uint32_t)cb * k, cb) : smem_desc(sb + 256u * k, K);
+        mma_bf16(tmem_d, da, db, idesc, (accumulate || k > 0) ? 1u : 0u);
+    }
+}
+
 // ---- tensor memory -> registers ---------------------------------------------
 // 32 consecutive FP32 columns of this thread's lane (32x32b shape, .x32).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
@@ -122,6 +153,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 4 consecutive FP32 columns (.x4).
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr)
+                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // TMEM address of (lane, column).
