@@ -236,6 +236,45 @@ __device__ __forceinline__ void warp_ranges_ball(const Geo& g, float px, float p
     }
 }
 
+// The candidate slots of a warp-uniform window, 32 at a time: f(slot) is called
+// by all lanes together, slot = -1 for lanes past the end, slots ascending over
+// the calls and lanes.  The lanes look up 32 columns at once and then take the
+// candidates of all of them in turn, so that a window of many short columns
+// (a few spheres each) costs one chain of loads per 32 candidates.
+template <class F>
+__device__ __forceinline__ void warp_candidates(const Geo& g, const Win& w, int inst, F&& f) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int ny = w.y1 - w.y0 + 1, ncols = w.x1 >= w.x0 && ny > 0 ? (w.x1 - w.x0 + 1) * ny : 0;
+    for (int c0 = 0; c0 < ncols; c0 += 32) {
+        const int c = c0 + lane;
+        int s = 0, n = 0;
+        if (c < ncols) {
+            const int base = inst * g.ncl + ((w.x0 + c / ny) * g.dim[1] + w.y0 + c % ny) * g.dim[2];
+            s = __ldg(g.start + base + w.z0);
+            n = max(0, __ldg(g.start + base + w.z1 + 1) - s);
+        }
+        int end = n;  // inclusive prefix sum
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kAll, end, o);
+            if (lane >= o) end += v;
+        }
+        const int total = __shfl_sync(kAll, end, 31);
+        const unsigned some = __ballot_sync(kAll, n > 0);
+        for (int u0 = 0; u0 < total; u0 += 32) {
+            const int u = u0 + lane;
+            int slot = -1;
+            for (unsigned m = some; m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const int ce = __shfl_sync(kAll, end, src), cn = __shfl_sync(kAll, n, src), cs = __shfl_sync(kAll, s, src);
+                if (u >= ce - cn && u < ce) slot = cs + (u - (ce - cn));
+            }
+            f(slot);
+        }
+    }
+}
+
 // Membership d2 < t for a candidate, exactly as the FP32 predicate with every
 // operation rounded, but decided from the cheaper contracted dot product
 // whenever it is clear of the bound: fma-contracted and fully rounded dot
