@@ -1,10 +1,13 @@
 """The warp-wide walks over the spheres at the sizes where they change shape:
-contact rows of no, a few, one warp's, and more contacts than the row buffer."""
+contact rows of no, a few, one warp's, and more contacts than the row buffer;
+crowds of spheres around a few fluid particles (several tiles of 32 spheres);
+the drag sums as a cluster of CTAs and as one CTA (more spheres than
+clusters are used for), which give the same bits."""
 import numpy as np
 import pytest
 import torch
 
-from helpers import field_err
+from helpers import field_err, scene
 from oracle.oracle import HostState
 from warp_sph_gpt_gb300 import HashGrid
 from warp_sph_gpt_gb300 import kernels as K
@@ -70,3 +73,46 @@ def test_contact_rows_of_every_length(m):
             assert int(D.contact_dem_offset_old[1]) == m and int(D.contact_bnd_offset_old[1]) == m
         assert field_err(_np(D.force), h64.dem["force"]) < TOL
         assert field_err(_np(D.torque), h64.dem["torque"]) < TOL
+
+
+@pytest.mark.parametrize("n_dem", [1, 33, 300])
+def test_coupling_with_crowds_of_spheres(n_dem):
+    s, P, B, _, _, grids = scene()
+    rng = np.random.default_rng(n_dem)
+    pos = rng.uniform([0.02, 0.02, 0.02], [0.38, 0.3, 0.5], (n_dem, 3))
+    D = _spheres(pos, rng.uniform(0.005, 0.02, n_dem), rng, 8)
+    P.vel.copy_(torch.tensor(rng.normal(0, 0.3, (P.n, 3)), dtype=torch.float32))
+    P.pres.copy_(torch.tensor(rng.uniform(0, 4e3, P.n), dtype=torch.float32))
+    grids[2].build(D.pos, 0.16)
+    h = HostState(P, B, D, None)
+    K.Kernel_prep_sphdem(P, B, D, *grids[:3], 0.16, 0.08, s.support, s.h, 0.05, 1.0)
+    K.Kernel_interaction_dem(P, D, grids[0], grids[2], s.mu, 0.05, 1.0, s.dt)
+    K.Kernel_interaction_sph(P, D, grids[0], grids[2], 0.16)
+    h.prep_sphdem(0.16, 0.08, s.support, s.h, 0.05, 1.0, p="f64")
+    h.interaction_dem(s.mu, 0.05, 1.0, s.dt, p="f64")
+    h.interaction_sph(0.16, p="f64")
+    assert field_err(_np(P.porosity), h.sph["porosity"]) < TOL
+    for name in ("flt_s", "porosity", "drag", "pressure_force"):
+        assert field_err(_np(getattr(D, name)), h.dem[name]) < TOL, name
+    assert field_err(_np(P.acc_dem), h.sph["acc_dem"]) < TOL
+
+
+def test_drag_sums_of_a_cluster_and_of_one_cta():
+    s, P, B, _, _, grids = scene()
+    rng = np.random.default_rng(3)
+    pos = rng.uniform([0.02, 0.02, 0.02], [0.38, 0.3, 0.5], (513, 3))
+    pos[8:] += [0.0, 0.0, 40.0]  # beyond the reach of the first eight and of the fluid
+    rad = np.full(513, 0.02)
+    P.vel.copy_(torch.tensor(rng.normal(0, 0.3, (P.n, 3)), dtype=torch.float32))
+    P.pgf.copy_(torch.tensor(rng.normal(0, 1.0, (P.n, 3)), dtype=torch.float32))
+    got = []
+    for n in (8, 513):
+        D = _spheres(pos[:n], rad[:n], np.random.default_rng(1), 8)
+        D.vel.zero_()
+        gd = HashGrid()
+        gd.build(D.pos, 0.16)
+        K.Kernel_interaction_dem(P, D, grids[0], gd, s.mu, 0.05, 1.0, s.dt)
+        got.append([_np(getattr(D, k))[:8] for k in ("flt_s", "porosity", "drag", "pressure_force")])
+    assert np.abs(got[0][2]).max() > 0
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a, b)

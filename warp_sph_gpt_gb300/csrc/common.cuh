@@ -214,16 +214,14 @@ struct MaskIter {
 // Warp-cooperative ball enumeration: the 32 lanes trim 32 columns at a time
 // (instead of every lane trimming every column), then f(s, e) is called
 // warp-uniformly for each non-empty range, in column order.
-// With part / parts, the warp takes only every parts-th batch of 32 columns
-// from batch `part` on (the warps of a CTA sharing one ball).
 template <class F>
 __device__ __forceinline__ void warp_ranges_ball(const Geo& g, float px, float py, float pz, float rq, int inst,
-                                                 F&& f, int part = 0, int parts = 1) {
+                                                 F&& f) {
     const int lane = threadIdx.x & 31;
     const Win w = window(g, px, py, pz, rq);
     const int ny = w.y1 - w.y0 + 1;
     const int ncols = (w.x1 - w.x0 + 1) * ny;
-    for (int c0 = 32 * part; c0 < ncols; c0 += 32 * parts) {
+    for (int c0 = 0; c0 < ncols; c0 += 32) {
         int s = 0, e = 0;
         const int c = c0 + lane;
         if (c < ncols) column_range_ball(g, w.x0 + c / ny, w.y0 + c % ny, px, py, pz, rq, inst, s, e);

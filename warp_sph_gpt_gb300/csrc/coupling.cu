@@ -9,15 +9,18 @@
 //   k_porosity_near   one warp per listed particle: the fluid normaliser as a
 //                     warp-strided sum over the coupling support, then the solid
 //                     fraction over the DEM neighbours.
-//   k_interaction_dem one CTA per DEM (Kernel_interaction_dem, :118-187): its
-//                     warps share the ball's columns; volume-weighted sums of
-//                     rho, u and -grad p reduced over the CTA in fixed order,
-//                     solid fraction, semi-implicit Ergun / Wen-Yu drag,
-//                     buoyancy.
+//   k_interaction_dem a cluster of 4 CTAs per DEM (Kernel_interaction_dem,
+//                     :118-187): its 32 warps share the ball's ranges; volume-
+//                     weighted sums of rho, u and -grad p and the solid
+//                     fraction reduced over the cluster in fixed order, semi-
+//                     implicit Ergun / Wen-Yu drag, buoyancy.
 //   k_react           Kernel_interaction_sph (:190-226) fused with
 //                     Kernel_step_sph (kernel/KERNEL_step.py:6-22).
 // Sums use fixed lane/warp orders, so every result is deterministic.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+#include "demwalk.cuh"
 #include "tma.cuh"
 
 namespace sd {
@@ -448,69 +451,99 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_porosity_tiles(CplArgs a) {
     }
 }
 
-constexpr int kIdThreads = 256;
+// Kernel_interaction_dem: kIdRanks x 8 warps per DEM a, the ranks as a cluster
+// of CTAs or one after another in one CTA (CTAS = kIdRanks or 1: the same sums
+// in the same order).  The fluid in a ball (2,000 to 140,000 particles) is a
+// few hundred slot ranges in batches of 32 columns; a task is a batch and
+// every per-th range of it.  One CTA whose 8 warps took whole batches needed
+// 58 us for 20 spheres at dx = 0.02 (two warps had columns at all) and 125 us
+// for 160 at 0.01: now 12 and 25 us.
+constexpr int kIdThreads = 256, kIdRanks = 4, kIdWarps = kIdThreads / 32 * kIdRanks;
+constexpr int kIdSums = 9;  // flt, rho_f, vel_f xyz, pgf xyz, solid
 
-// Kernel_interaction_dem: one CTA per DEM a.
+template <int CTAS>
 __global__ void __launch_bounds__(kIdThreads) k_interaction_dem(CplArgs a) {
     pdl_wait();
     pdl_launch();
-    __shared__ float red[kIdThreads / 32][8];
-    const int am = blockIdx.x;
+    namespace cg = cooperative_groups;
+    __shared__ float red[kIdThreads / 32][kIdSums];
+    __shared__ float sums[kIdRanks][kIdSums];
+    constexpr unsigned kAll = 0xffffffffu;
+    const int am = blockIdx.x / CTAS, cta = blockIdx.x % CTAS, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float3 pa = ld3(a.D.pos, am);
     const float4 aux = a.aux[am];  // 1/h, cw, bound(2h), 2h
     const int inst = inst_of(a.gd, am);
-    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // flt, rho_f, vel_f xyz, pgf xyz
-    if (a.P.n > 0) {
-        // the warps take turns at 32-column batches of the ball and their
-        // lanes stride through each range (ranges are ~10x longer than a warp
-        // and mostly shorter than the CTA)
-        const float t_lo = band_lo(aux.z), t_hi = band_hi(aux.z);
-        const int lane = threadIdx.x & 31;
-        warp_ranges_ball(a.gs, pa.x, pa.y, pa.z, pad_radius(aux.w), inst, [&](int rs, int re) {
-            for (int j = rs + lane; j < re; j += 32) {
-                const float4 q = a.f_posv[j];
-                float d2;
-                if (d2_below(pa.x - q.x, pa.y - q.y, pa.z - q.z, t_lo, t_hi, aux.z, d2)) {  // len < 2 h_a, :157-158
-                    const float Vw = q.w * w_aux(aux, fast_sqrt(d2));
-                    const float4 v = a.f_vel[j];
-                    const float4 g = a.f_pgf[j];
-                    s[0] += Vw;
-                    s[1] += g.w * Vw;
-                    s[2] += v.x * Vw;
-                    s[3] += v.y * Vw;
-                    s[4] += v.z * Vw;
-                    s[5] += g.x * Vw;
-                    s[6] += g.y * Vw;
-                    s[7] += g.z * Vw;
+    const float rq = pad_radius(aux.w);
+    const float t_lo = band_lo(aux.z), t_hi = band_hi(aux.z);
+    const Win w = window(a.gs, pa.x, pa.y, pa.z, rq);
+    const int ny = w.y1 - w.y0 + 1, ncols = a.P.n > 0 ? (w.x1 - w.x0 + 1) * ny : 0, batches = (ncols + 31) / 32;
+    int per = 1;  // tasks per batch
+    while (per < 16 && per * batches < 2 * kIdWarps) per *= 2;
+    float s[kIdSums];
+#pragma unroll 1
+    for (int rank = cta; rank < kIdRanks; rank += CTAS) {
+        const int me = rank * (kIdThreads / 32) + wid;
+#pragma unroll
+        for (int c = 0; c < kIdSums; ++c) s[c] = 0.0f;
+        for (int task = me; task < per * batches; task += kIdWarps) {
+            const int c = 32 * (task / per) + lane;
+            int rs = 0, re = 0;
+            if (c < ncols) column_range_ball(a.gs, w.x0 + c / ny, w.y0 + c % ny, pa.x, pa.y, pa.z, rq, inst, rs, re);
+            const unsigned some = __ballot_sync(kAll, re > rs);
+            const int turn = __popc(some & ((1u << lane) - 1u)) % per;
+            for (unsigned mine = __ballot_sync(kAll, re > rs && turn == task % per); mine; mine &= mine - 1) {
+                const int src = __ffs(mine) - 1;
+                const int j0 = __shfl_sync(kAll, rs, src), j1 = __shfl_sync(kAll, re, src);
+#pragma unroll 2
+                for (int j = j0 + lane; j < j1; j += 32) {
+                    const float4 q = a.f_posv[j], v = a.f_vel[j], g = a.f_pgf[j];
+                    float d2;
+                    if (d2_below(pa.x - q.x, pa.y - q.y, pa.z - q.z, t_lo, t_hi, aux.z, d2)) {  // len < 2 h_a, :157-158
+                        const float Vw = q.w * w_aux(aux, fast_sqrt(d2));
+                        s[0] += Vw;
+                        s[1] += g.w * Vw;
+                        s[2] += v.x * Vw;
+                        s[3] += v.y * Vw;
+                        s[4] += v.z * Vw;
+                        s[5] += g.x * Vw;
+                        s[6] += g.y * Vw;
+                        s[7] += g.z * Vw;
+                    }
                 }
             }
-        }, threadIdx.x >> 5, kIdThreads / 32);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const float v = warp_sum(s[c]);
-        if (lane == 0) red[wid][c] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int c = 0; c < 8; ++c) {
-        float t = 0.0f;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[k][c];
-        s[c] = t;
-    }
-    // solid sum over DEM neighbours, a itself included (:165-168)
-    float solid = 0.0f;
-    const Win wd = window(a.gd, pa.x, pa.y, pa.z, pad_radius(aux.w));
-    for_each_range(a.gd, wd, inst, [&](int rs, int re) {
-        for (int j = rs; j < re; ++j) {
-            const int b = a.gd.order[j];
+        }
+        // solid sum over DEM neighbours, a itself included (:165-168)
+        int chunk = 0;
+        warp_candidates(a.gd, window(a.gd, pa.x, pa.y, pa.z, rq), inst, [&](int slot) {
+            if (chunk++ % kIdWarps != me || slot < 0) return;
+            const int b = a.gd.order[slot];
             const float3 pb = ld3(a.D.pos, b);
             const D2 r = d2_exact(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-            if (r.d2 < aux.z) solid += a.D.volume[b] * w_aux(aux, fast_sqrt(r.d2));
+            if (r.d2 < aux.z) s[8] += a.D.volume[b] * w_aux(aux, fast_sqrt(r.d2));
+        });
+#pragma unroll
+        for (int c = 0; c < kIdSums; ++c) {
+            const float v = warp_sum(s[c]);
+            if (lane == 0) red[wid][c] = v;
         }
-    });
-    const float flt = s[0];
+        __syncthreads();
+        if (threadIdx.x < kIdSums) {
+            float t = 0.0f;
+            for (int k = 0; k < kIdThreads / 32; ++k) t += red[k][threadIdx.x];
+            float* first = &sums[0][0];
+            if (CTAS > 1) first = cg::this_cluster().map_shared_rank(first, 0);
+            first[rank * kIdSums + threadIdx.x] = t;
+        }
+        __syncthreads();
+    }
+    if (CTAS > 1) cg::this_cluster().sync();
+    if (cta != 0 || threadIdx.x != 0) return;
+    for (int c = 0; c < kIdSums; ++c) {
+        float t = 0.0f;
+        for (int k = 0; k < kIdRanks; ++k) t += sums[k][c];
+        s[c] = t;
+    }
+    const float flt = s[0], solid = s[8];
     a.D.flt_s[am] = flt;
     float3 drag = make_float3(0.f, 0.f, 0.f), pf = make_float3(0.f, 0.f, 0.f);
     float por = a.eps_max;
@@ -536,35 +569,38 @@ __global__ void __launch_bounds__(kIdThreads) k_interaction_dem(CplArgs a) {
     st3(a.D.pressure_force, am, pf);
 }
 
-// Kernel_interaction_sph (+ Kernel_step_sph when INTEGRATE), point order.
+// Kernel_interaction_sph (+ Kernel_step_sph when INTEGRATE), grid order: the
+// particles of a warp share their spheres (demwalk.cuh).
+constexpr int kReactThreads = 128;
 template <bool INTEGRATE>
-__global__ void k_react(CplArgs a) {
+__global__ void __launch_bounds__(kReactThreads) k_react(CplArgs a) {
     pdl_wait();
     pdl_launch();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.P.n) return;
-    const float3 pi = ld3(a.P.pos, i);
+    __shared__ DemTile tiles[kReactThreads / 32];
+    DemTile& sh = tiles[threadIdx.x >> 5];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool mine = k < a.P.n;
+    const int i = mine ? a.gs.order[k] : 0;
+    const float3 pi = mine ? ld3(a.P.pos, i) : make_float3(0.f, 0.f, 0.f);
     float3 fd = make_float3(0.f, 0.f, 0.f);
-    if (a.D.n > 0) {
-        const int inst = inst_of(a.gs, i);
-        const Win w = window(a.gd, pi.x, pi.y, pi.z, a.rq);
-        for_each_range(a.gd, w, inst, [&](int s, int e) {
-            for (int j = s; j < e; ++j) {
-                const int b = a.gd.order[j];
-                const float3 pb = ld3(a.D.pos, b);
-                const D2 r = d2_exact(pi.x, pi.y, pi.z, pb.x, pb.y, pb.z);
-                const float4 ab = a.aux[b];
+    if (a.D.n > 0)
+        warp_dem_visit(
+            a.gd, mine, pi.x, pi.y, pi.z, a.rq, mine ? inst_of(a.gs, i) : 0, sh,
+            [&](int b, float4& p, float4& q, float4& r) {
+                const float3 x = ld3(a.D.pos, b), dr = ld3(a.D.drag, b);
                 const float flt_s = a.D.flt_s[b];
-                if (r.d2 < ab.z && flt_s > 1.0e-12f) {  // :220-221
-                    const float c = w_aux(ab, fast_sqrt(r.d2)) / flt_s;
-                    const float3 dr = ld3(a.D.drag, b);
-                    fd.x -= dr.x * c;
-                    fd.y -= dr.y * c;
-                    fd.z -= dr.z * c;
-                }
-            }
-        });
-    }
+                q = a.aux[b];
+                p = make_float4(x.x, x.y, x.z, flt_s > 1.0e-12f ? q.z : -1.0f);  // :220-221
+                r = make_float4(dr.x, dr.y, dr.z, flt_s);
+            },
+            [&](int t, float d2) {
+                const float4 dr = sh.r[t];
+                const float c = w_aux(sh.q[t], fast_sqrt(d2)) / dr.w;
+                fd.x -= dr.x * c;
+                fd.y -= dr.y * c;
+                fd.z -= dr.z * c;
+            });
+    if (!mine) return;
     const float den = a.P.rho[i] * a.P.porosity[i];
     const float3 acc_dem = make_float3(fd.x / den, fd.y / den, fd.z / den);
     st3(a.P.acc_dem, i, acc_dem);
@@ -573,6 +609,8 @@ __global__ void k_react(CplArgs a) {
     st3(a.P.acc, i, acc);
     if (INTEGRATE) euler_store(a.P.pos, a.P.vel, i, acc, a.dt);
 }
+
+constexpr int kIdClusterMax = 512;
 
 CplArgs make_args(const sphdem_ctx_t* c, float support, float h) {
     CplArgs a;
@@ -653,7 +691,26 @@ int run_interaction_dem(const sphdem_ctx_t* c, float mu, float eps_min, float ep
     a.eps_min = eps_min;
     a.eps_max = eps_max;
     a.dt = dt;
-    launch_pdl(k_interaction_dem, c->dem.n, kIdThreads, 0, st, a);
+    // a cluster per sphere while that leaves CTAs to spare: 2,000 spheres, most
+    // of them dry, took 339 us as clusters that each worked out all columns in
+    // every warp, and 168 as whole batches per warp
+    if (c->dem.n > kIdClusterMax) {
+        launch_pdl(k_interaction_dem<1>, c->dem.n, kIdThreads, 0, st, a);
+    } else {
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = kIdRanks;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kIdRanks * c->dem.n);
+        cfg.blockDim = dim3(kIdThreads);
+        cfg.stream = st;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        cudaLaunchKernelEx(&cfg, k_interaction_dem<kIdRanks>, a);  // errors surface through launch_status
+    }
     return launch_status("interaction_dem");
 }
 
@@ -663,9 +720,9 @@ int run_react(const sphdem_ctx_t* c, float support, float dt, bool integrate, cu
     CplArgs a = make_args(c, support, 0.0f);
     a.dt = dt;
     if (integrate)
-        launch_pdl(k_react<true>, blocks_for(n, 256), 256, 0, st, a);
+        launch_pdl(k_react<true>, blocks_for(n, kReactThreads), kReactThreads, 0, st, a);
     else
-        launch_pdl(k_react<false>, blocks_for(n, 256), 256, 0, st, a);
+        launch_pdl(k_react<false>, blocks_for(n, kReactThreads), kReactThreads, 0, st, a);
     return launch_status("react");
 }
 

@@ -36,7 +36,7 @@
 // candidates of a tile's wider window change nothing.
 //
 // Kernels (one porosity pass):
-//   k_pnear      one thread per fluid slot: a DEM within 2 h_b?  Dry particles
+//   k_pnear      a warp per 32 fluid slots: a DEM within 2 h_b?  Dry particles
 //                get clamp(1); listed ones are counted per frame block, and a
 //                frame block's first listed particle puts it on a list.
 //   k_plist      one warp per listed frame block: reserves its segment of the
@@ -49,7 +49,7 @@
 //                and owns tensor memory, warps 9-10 stage candidate rows
 //                (each thread loads its next chunk's candidates while it
 //                builds the current chunk's rows).
-//   k_pfinish    one thread per listed particle: slab partials -> flt, solid
+//   k_pfinish    a warp per 32 listed particles: slab partials -> flt, solid
 //                fraction over the DEM neighbours, porosity.
 // Every wait is bounded; a timeout raises SPHDEM_FLAG_TIMEOUT, the CTA drains
 // its MMAs (bounded) and frees its tensor memory.
@@ -60,6 +60,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "demwalk.cuh"
 #include "umma.cuh"
 
 namespace sd {
@@ -209,27 +210,28 @@ __device__ __forceinline__ void frame_cells(const PorArgs& a, int d, int f, int&
 // ---------------------------------------------------------------------------
 // near flags, dry particles, per-frame-block counts
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_pnear(PorArgs a) {
+constexpr int kNearThreads = 128;
+
+__global__ void __launch_bounds__(kNearThreads) k_pnear(PorArgs a) {
     pdl_wait();
     pdl_launch();
+    __shared__ DemTile tiles[kNearThreads / 32];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.P.n) return;
-    const int o = a.gs.order[k];
-    const float4 p = a.f_posm[k];  // positions only: runs before the density pass is done
-    const int key = a.gs.key[o];
+    const bool mine = k < a.P.n;
+    const int o = mine ? a.gs.order[k] : 0;
+    const float4 p = mine ? a.f_posm[k] : make_float4(0.f, 0.f, 0.f, 0.f);  // positions only: runs before the density pass is done
+    const int key = mine ? a.gs.key[o] : 0;
     const int inst = a.gs.ncl > 0 ? key / a.gs.ncl : 0;
     bool near = false;
-    if (a.D.n > 0) {
-        const Win w = window(a.gd, p.x, p.y, p.z, a.rq);
-        for_each_range(a.gd, w, inst, [&](int s, int e) {
-            for (int j = s; j < e && !near; ++j) {
-                const int b = a.gd.order[j];
-                const float3 pb = ld3(a.D.pos, b);
-                const D2 r = d2_exact(p.x, p.y, p.z, pb.x, pb.y, pb.z);
-                if (r.d2 < a.aux[b].z) near = true;  // len < 2 h_b, :87-88
-            }
-        });
-    }
+    if (a.D.n > 0)
+        warp_dem_visit(
+            a.gd, mine, p.x, p.y, p.z, a.rq, inst, tiles[threadIdx.x >> 5],
+            [&](int b, float4& q, float4&, float4&) {
+                const float3 x = ld3(a.D.pos, b);
+                q = make_float4(x.x, x.y, x.z, a.aux[b].z);  // len < 2 h_b, :87-88
+            },
+            [&](int, float) { near = true; });
+    if (!mine) return;
     a.flag[k] = near ? 1 : 0;
     if (near) {
         const int local = key - inst * a.gs.ncl;
@@ -706,37 +708,42 @@ __global__ void __launch_bounds__(kPThreads, 2) k_porosity_mma(PorArgs a) {
 // ---------------------------------------------------------------------------
 // slab partials -> normaliser -> solid fraction -> porosity
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_pfinish(PorArgs a) {
+__global__ void __launch_bounds__(kNearThreads) k_pfinish(PorArgs a) {
     pdl_wait();
     pdl_launch();
+    __shared__ DemTile tiles[kNearThreads / 32];
+    DemTile& sh = tiles[threadIdx.x >> 5];
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= a.ctl->n_near) return;
-    const int k = a.near_list[idx];
+    const int n_near = a.ctl->n_near;
+    if ((idx & ~31) >= n_near) return;  // the warp has no entry
+    const bool mine = idx < n_near;
+    const int k = mine ? a.near_list[idx] : 0;
     const int o = a.gs.order[k];
     float f = 0.0f;
+    if (mine)
 #pragma unroll
-    for (int s = 0; s < kPSlabs; ++s) f += a.part[(size_t)idx * kPSlabs + s];
+        for (int s = 0; s < kPSlabs; ++s) f += a.part[(size_t)idx * kPSlabs + s];
     const float flt = f * a.cw;
     const float4 p = a.f_posv[k];
     const int inst = a.gs.ncl > 0 ? a.gs.key[o] / a.gs.ncl : 0;
     float solid = 0.0f;
-    const Win w = window(a.gd, p.x, p.y, p.z, a.rq);
-    for_each_range(a.gd, w, inst, [&](int s, int e) {
-        for (int j = s; j < e; ++j) {
-            const int b = a.gd.order[j];
+    warp_dem_visit(
+        a.gd, mine, p.x, p.y, p.z, a.rq, inst, sh,
+        [&](int b, float4& x, float4& q, float4&) {
             const float3 pb = ld3(a.D.pos, b);
-            const D2 r = d2_exact(p.x, p.y, p.z, pb.x, pb.y, pb.z);
             const float4 ab = a.aux[b];
-            if (r.d2 < ab.z) {  // len < 2 h_b, :87-88
-                const float q = fast_sqrt(r.d2) * ab.x;
-                const float uu = 1.0f - 0.5f * q;
-                const float u2 = uu * uu;
-                const float wb = q < 2.0f ? ab.y * u2 * u2 * (1.0f + 2.0f * q) : 0.0f;
-                solid += a.D.volume[b] * wb / (flt + 1.0e-20f);
-            }
-        }
-    });
-    a.P.porosity[o] = fminf(fmaxf(1.0f - solid, a.eps_min), a.eps_max);
+            x = make_float4(pb.x, pb.y, pb.z, ab.z);  // len < 2 h_b, :87-88
+            q = make_float4(ab.x, ab.y, a.D.volume[b], 0.0f);
+        },
+        [&](int t, float d2) {
+            const float4 ab = sh.q[t];
+            const float q = fast_sqrt(d2) * ab.x;
+            const float uu = 1.0f - 0.5f * q;
+            const float u2 = uu * uu;
+            const float wb = q < 2.0f ? ab.y * u2 * u2 * (1.0f + 2.0f * q) : 0.0f;
+            solid += ab.z * wb / (flt + 1.0e-20f);
+        });
+    if (mine) a.P.porosity[o] = fminf(fmaxf(1.0f - solid, a.eps_min), a.eps_max);
 }
 
 // Frame-block lattice of the fluid grid (world-anchored), per axis.
@@ -841,12 +848,12 @@ int run_porosity_mma(const sphdem_ctx_t* c, float support, float h, float eps_mi
             set_error("porosity memset", e);
             return SPHDEM_ERR_CUDA;
         }
-        launch_pdl(k_pnear, blocks_for(n, 256), 256, 0, st, a);
+        launch_pdl(k_pnear, blocks_for(n, kNearThreads), kNearThreads, 0, st, a);
         launch_pdl(k_plist, 8 * sms, 256, 0, st, a);
     }
     if (part != 1) {
         launch_pdl(k_porosity_mma, 2 * sms, kPThreads, kPSmemBytes, st, a);
-        launch_pdl(k_pfinish, blocks_for(n, 256), 256, 0, st, a);
+        launch_pdl(k_pfinish, blocks_for(n, kNearThreads), kNearThreads, 0, st, a);
     }
     return launch_status("porosity (tensor cores)");
 }

@@ -76,12 +76,6 @@ __device__ __forceinline__ void visit_members(const Geo& g, const float4* __rest
     }
 }
 
-// Adds a b of this lane (0 if !ok) to the subject's sum.
-template <int LANES>
-__device__ __forceinline__ float lanes_fma(float acc, float a, float b) {
-    return LANES == 1 || LANES == 32 ? fmaf(a, b, acc) : ordered_fma<LANES == 32 ? 1 : LANES>(acc, a, b);
-}
-
 template <int LANES>
 __device__ __forceinline__ float lanes_sum(float v) {
     return LANES == 32 ? warp_sum(v) : v;
@@ -178,30 +172,39 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
     } else {
         const bool list = LANES != 32 && a.nbr != nullptr;
         const int shift = (threadIdx.x & 31) - lane;  // first lane of this subject
-        int found = 0;                                // members so far (recorded in rows, up to the capacity)
-        const float* __restrict__ vprev = a.f_vprev;
-        int32_t* rows = a.nbr;
-        auto member = [&](bool ok, int j, const float4& q, const D2& r) {
-            const float w = ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f;
-            if (list && LANES == 1) {
-                if (found < a.cap) rows[(size_t)found * n + k] = j;
-                ++found;
-            } else if (list) {
-                const unsigned of = (__ballot_sync(0xffffffffu, ok) >> shift) & ((1u << (LANES & 31)) - 1u);
-                const int row = found + __popc(of & ((1u << lane) - 1u));
-                if (ok && row < a.cap) rows[(size_t)row * n + k] = j;
-                found += __popc(of);
-            }
-            if (RHO) rho_sum = lanes_fma<LANES>(rho_sum, ok ? q.w : 0.0f, w);
-            if (FLT) flt_sum = lanes_fma<LANES>(flt_sum, ok ? vprev[j] : 0.0f, w);
+        // one kind's members: sums, and their slots into rows, up to the capacity
+        auto kind = [&](const Geo& g, const float4* __restrict__ posm, const float* __restrict__ vprev, int first_row,
+                        int count_row) {
+            int found = 0;
+            visit_members<LANES>(g, posm, mine, p, a.rq, a.s2, inst, lane, [&](bool ok, int j, const float4& q,
+                                                                              const D2& r) {
+                if constexpr (LANES == 1 || LANES == 32) {
+                    const float w = kern_w(a.kern, fast_sqrt(r.d2));
+                    if (RHO) rho_sum += q.w * w;
+                    if (FLT) flt_sum += vprev[j] * w;
+                    if (list) {
+                        if (found < a.cap) a.nbr[(size_t)(first_row + found) * n + k] = j;
+                        ++found;
+                    }
+                } else {
+                    const float w = ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f;
+                    if (list) {
+                        const unsigned of = (__ballot_sync(0xffffffffu, ok) >> shift) & ((1u << (LANES & 31)) - 1u);
+                        const int row = found + __popc(of & ((1u << lane) - 1u));
+                        if (ok && row < a.cap) a.nbr[(size_t)(first_row + row) * n + k] = j;
+                        found += __popc(of);
+                    }
+                    if (RHO) rho_sum = ordered_fma<LANES>(rho_sum, ok ? q.w : 0.0f, w);
+                    if (FLT) flt_sum = ordered_fma<LANES>(flt_sum, ok ? vprev[j] : 0.0f, w);
+                }
+            });
+            if (list && mine && lane == 0) a.nbr[(size_t)count_row * n + k] = found;
         };
-        visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane, member);
-        if (list && mine && lane == 0) a.nbr[(size_t)(2 * a.cap) * n + k] = found;
-        found = 0;
-        vprev = a.b_vprev;
-        rows += (size_t)a.cap * n;
-        if (a.gb.ncl > 0) visit_members<LANES>(a.gb, a.b_posm, mine, p, a.rq, a.s2, inst, lane, member);
-        if (list && mine && lane == 0) a.nbr[(size_t)(2 * a.cap + 1) * n + k] = found;
+        kind(a.gs, a.f_posm, a.f_vprev, 0, 2 * a.cap);
+        if (a.gb.ncl > 0)
+            kind(a.gb, a.b_posm, a.b_vprev, a.cap, 2 * a.cap + 1);
+        else if (list && mine && lane == 0)
+            a.nbr[(size_t)(2 * a.cap + 1) * n + k] = 0;
     }
     if (RHO) rho_sum = lanes_sum<LANES>(rho_sum);
     if (FLT) flt_sum = lanes_sum<LANES>(flt_sum);
@@ -250,8 +253,11 @@ __global__ void __launch_bounds__(256) k_density_wall(WallArgs a) {
     if (a.gs.ncl > 0)
         visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane,
                              [&](bool ok, int j, const float4& q, const D2& r) {
-                                 const float w = ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f;
-                                 rho_sum = lanes_fma<LANES>(rho_sum, ok ? q.w : 0.0f, w);
+                                 if constexpr (LANES == 1 || LANES == 32)
+                                     rho_sum += q.w * kern_w(a.kern, fast_sqrt(r.d2));
+                                 else
+                                     rho_sum = ordered_fma<LANES>(rho_sum, ok ? q.w : 0.0f,
+                                                                  ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f);
                              });
     rho_sum = lanes_sum<LANES>(rho_sum);
     if (lane != 0 || !mine) return;
