@@ -12,10 +12,10 @@
 // 128 subjects against a chunk of 128 candidates come from one tcgen05 MMA:
 //     s_ij = |p_i|^2 + |q_j|^2 - 2 p_i . q_j
 // with p, q in units of h relative to a common centre, every FP32 operand
-// split exactly into three BF16 pieces (a = a0 + a1 + a2) and the six
-// significant products of p . q, plus the pieces of |p|^2 and |q|^2 times
-// ones, laid along K = 32: the FP32 accumulation of exact BF16 products gives
-// s to ~1e-6 of the ball radius squared.  The CUDA cores then evaluate only
+// split exactly into three BF16 pieces (a = a0 + a1 + a2) and all products of
+// p . q but p2 q2 (below 2^-32 of |p| |q|), plus the pieces of |p|^2 and |q|^2
+// times ones, laid along K = 32: the FP32 accumulation of exact BF16 products
+// gives s to ~1e-6 of the ball radius squared.  The CUDA cores then evaluate only
 // w(s) (one MUFU square root, the polynomial on packed FP32 pairs) and the
 // V_j-weighted sums.
 //
@@ -41,20 +41,19 @@
 //                frame block's first listed particle puts it on a list.
 //   k_plist      one warp per listed frame block: reserves its segment of the
 //                near list and of the tile table (atomics: segment placement
-//                varies, results do not), writes its listed slots by 2 x 2 x 2
-//                cell sub-blocks (so a tile of 128 is compact) and its tiles.
+//                varies, results do not), writes its listed slots along
+//                pencils of 2 x 2 cells (so a tile of 128 is compact) and its
+//                tiles.
 //   k_porosity_mma  persistent, 2 CTAs per SM: work units (tile, slab);
 //                warps 0-7 epilogue (TMEM lane = subject; warp w reads lane
-//                quarter w mod 4, chunk half w / 4), warp 8 issues the MMAs
-//                and owns tensor memory, warps 9-10 stage candidate rows
-//                (each thread loads its next chunk's candidates while it
-//                builds the current chunk's rows).
+//                quarter w mod 4, chunk half w / 4), warps 8-11 stage
+//                candidate rows (each thread loads its next chunk's candidate
+//                while it builds the current chunk's row); warp 8 also issues
+//                the MMAs and owns tensor memory.
 //   k_pfinish    a warp per 32 listed particles: slab partials -> flt, solid
 //                fraction over the DEM neighbours, porosity.
 // Every wait is bounded; a timeout raises SPHDEM_FLAG_TIMEOUT, the CTA drains
 // its MMAs (bounded) and frees its tensor memory.
-#include <cuda_bf16.h>
-
 #include <map>
 #include <mutex>
 #include <utility>
@@ -69,16 +68,15 @@ namespace {
 
 constexpr int kPM = 128;            // subjects per tile (MMA M, TMEM lanes)
 constexpr int kPN = 128;            // candidates per chunk (MMA N, TMEM columns)
-constexpr int kPK = 32;             // BF16 K of the distance MMA (24 used)
+constexpr int kPK = 32;             // BF16 K of the distance MMA (30 used)
 constexpr int kPStages = 6;         // candidate-row stages in shared memory
 constexpr int kPSlabs = SPHDEM_POROSITY_SLABS;
 constexpr int kPMaxRanges = 512;    // candidate ranges per column batch
 constexpr int kPMaxChunks = 2048;   // chunks per column batch with a precomputed first range
 constexpr int kPEpiWarps = 8;       // two per TMEM lane quarter, one per half of each chunk
-constexpr int kPMmaWarp = 8;
-constexpr int kPStageWarps = 2;
-constexpr int kPThreads = 32 * (kPEpiWarps + 1 + kPStageWarps);  // 352
-constexpr int kPStageThreads = 32 * kPStageWarps;
+constexpr int kPStageWarps = 4;     // one thread per candidate of a chunk; the first also issues the MMAs
+constexpr int kPMmaWarp = kPEpiWarps;
+constexpr int kPThreads = 32 * (kPEpiWarps + kPStageWarps);  // 384
 constexpr int kPAlign = 8;          // candidate class = slot offset in the instance mod 8
 constexpr uint32_t kPRowBytes = kPK * 2;
 constexpr uint32_t kPTileBytes = kPM * kPRowBytes;  // = kPN * kPRowBytes
@@ -135,61 +133,55 @@ __device__ __forceinline__ float sqrt_apx(float x) {
     return r;
 }
 
-// Exact three-piece BF16 split of an FP32 value: a = a0 + a1 + a2.
-__device__ __forceinline__ void split3(float a, float& a0, float& a1, float& a2) {
-    a0 = __bfloat162float(__float2bfloat16_rn(a));
-    const float r1 = a - a0;
-    a1 = __bfloat162float(__float2bfloat16_rn(r1));
-    a2 = __bfloat162float(__float2bfloat16_rn(r1 - a1));
+// Exact three-piece BF16 split of an FP32 value, a = a0 + a1 + a2, by truncation
+// (8 of its 24 significant bits each): the bits of a piece are a float's upper
+// half, so a pair of them is one byte permute.  (Pieces rounded by conversion
+// instructions, two per piece and one per pair, made a row twice as long and
+// kept the unit busy that the square roots need: with two staging warps and
+// those, 3.00 ms at 800k and 0.99 at 100k with submerged spheres; with four
+// staging warps and this, 2.71 and 0.90.)
+__device__ __forceinline__ void split3(float a, uint32_t* t) {
+    t[0] = __float_as_uint(a) & 0xffff0000u;
+    const float r1 = a - __uint_as_float(t[0]);
+    t[1] = __float_as_uint(r1) & 0xffff0000u;
+    t[2] = __float_as_uint(r1 - __uint_as_float(t[1]));
 }
 
-__device__ __forceinline__ uint32_t pk(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);  // exact: both already BF16 values
-    return *reinterpret_cast<uint32_t*>(&h);
+// BF16 pair (lo, hi) of two pieces.
+__device__ __forceinline__ uint32_t pk(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x7632); }
+
+// One 64-byte operand row (32 BF16 along K) at row r of a K-major tile, from
+// the pieces of x, y, z and of the square n.  K holds per coordinate the
+// products a0b0, a0b1, a1b0, a0b2, a1b1, a2b0, a1b2, a2b1, with n against ones
+// on either side; SUBJECT: the a (and n before ones), else the b.
+template <bool SUBJECT>
+__device__ __forceinline__ void store_row(uint8_t* tile, int r, const uint32_t (*x)[3], const uint32_t* n) {
+    constexpr int i1 = SUBJECT ? 0 : 1, i2 = SUBJECT ? 1 : 0, i3 = SUBJECT ? 0 : 2, i5 = SUBJECT ? 2 : 0;
+    constexpr uint32_t kOne = 0x3f800000u;
+    const uint32_t m0 = SUBJECT ? n[0] : kOne, m1 = SUBJECT ? n[1] : kOne, m2 = SUBJECT ? n[2] : kOne;
+    const uint32_t l0 = SUBJECT ? kOne : n[0], l1 = SUBJECT ? kOne : n[1], l2 = SUBJECT ? kOne : n[2];
+    auto put = [&](int k, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+        *reinterpret_cast<uint4*>(tile + umma::tile_off(r, k, kPK)) = make_uint4(a, b, c, d);
+    };
+    // (x y z) of a0b0, a0b1, a1b0, a0b2, a1b1, a2b0, then n, then a1b2, a2b1
+    put(0, pk(x[0][0], x[1][0]), pk(x[2][0], x[0][i1]), pk(x[1][i1], x[2][i1]), pk(x[0][i2], x[1][i2]));
+    put(8, pk(x[2][i2], x[0][i3]), pk(x[1][i3], x[2][i3]), pk(x[0][1], x[1][1]), pk(x[2][1], x[0][i5]));
+    put(16, pk(x[1][i5], x[2][i5]), pk(m0, m1), pk(m2, l0), pk(l1, l2));
+    constexpr int i6 = SUBJECT ? 1 : 2, i7 = SUBJECT ? 2 : 1;
+    put(24, pk(x[0][i6], x[1][i6]), pk(x[2][i6], x[0][i7]), pk(x[1][i7], x[2][i7]), 0u);
 }
 
-// One 64-byte operand row (32 BF16 along K) at row r of a K-major tile:
-// v[0..23] the used columns, 24..31 zero.
-__device__ __forceinline__ void store_row(uint8_t* tile, int r, const float* v) {
-    uint4 w0 = make_uint4(pk(v[0], v[1]), pk(v[2], v[3]), pk(v[4], v[5]), pk(v[6], v[7]));
-    uint4 w1 = make_uint4(pk(v[8], v[9]), pk(v[10], v[11]), pk(v[12], v[13]), pk(v[14], v[15]));
-    uint4 w2 = make_uint4(pk(v[16], v[17]), pk(v[18], v[19]), pk(v[20], v[21]), pk(v[22], v[23]));
-    *reinterpret_cast<uint4*>(tile + umma::tile_off(r, 0, kPK)) = w0;
-    *reinterpret_cast<uint4*>(tile + umma::tile_off(r, 8, kPK)) = w1;
-    *reinterpret_cast<uint4*>(tile + umma::tile_off(r, 16, kPK)) = w2;
-    *reinterpret_cast<uint4*>(tile + umma::tile_off(r, 24, kPK)) = make_uint4(0, 0, 0, 0);
-}
-
-// Subject row: p pieces against -2 q pieces (p0q0, p0q1, p1q0, p0q2, p1q1,
-// p2q0 per coordinate), |p|^2 pieces against ones, ones against |q|^2 pieces.
-__device__ __forceinline__ void subject_row(float px, float py, float pz, float* v) {
-    float x[3][3];
-    split3(px, x[0][0], x[0][1], x[0][2]);
-    split3(py, x[1][0], x[1][1], x[1][2]);
-    split3(pz, x[2][0], x[2][1], x[2][2]);
-    const float pp = fmaf(pz, pz, fmaf(py, py, px * px));
-    const int pa[6] = {0, 0, 1, 0, 1, 2};
-#pragma unroll
-    for (int g = 0; g < 6; ++g)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) v[3 * g + d] = x[d][pa[g]];
-    split3(pp, v[18], v[19], v[20]);
-    v[21] = v[22] = v[23] = 1.0f;
-}
-
-__device__ __forceinline__ void candidate_row(float qx, float qy, float qz, float* v) {
-    float x[3][3];
-    split3(-2.0f * qx, x[0][0], x[0][1], x[0][2]);
-    split3(-2.0f * qy, x[1][0], x[1][1], x[1][2]);
-    split3(-2.0f * qz, x[2][0], x[2][1], x[2][2]);
-    const float qq = fmaf(qz, qz, fmaf(qy, qy, qx * qx));
-    const int pb[6] = {0, 1, 0, 2, 1, 0};
-#pragma unroll
-    for (int g = 0; g < 6; ++g)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) v[3 * g + d] = x[d][pb[g]];
-    v[18] = v[19] = v[20] = 1.0f;
-    split3(qq, v[21], v[22], v[23]);
+// Subject row: p pieces, |p|^2 pieces against ones, ones against |q|^2 pieces;
+// candidate row: -2 q pieces, ones, |q|^2 pieces.
+template <bool SUBJECT>
+__device__ __forceinline__ void make_row(uint8_t* tile, int r, float px, float py, float pz) {
+    uint32_t x[3][3], n[3];
+    const float f = SUBJECT ? 1.0f : -2.0f;
+    split3(f * px, x[0]);
+    split3(f * py, x[1]);
+    split3(f * pz, x[2]);
+    split3(fmaf(pz, pz, fmaf(py, py, px * px)), n);
+    store_row<SUBJECT>(tile, r, x, n);
 }
 
 // Frame block of local cell (cx, cy, cz) of instance inst.
@@ -245,11 +237,17 @@ __global__ void __launch_bounds__(kNearThreads) k_pnear(PorArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// listed slots of each frame block by sub-blocks of 2 x 2 x 2 cells, and its tiles
+// listed slots of each frame block, and its tiles: the cells in pencils of 2 x 2
+// columns, up one pencil and down the next, so that 128 consecutive particles
+// (7 cells) lie in a box of about 2 x 2 x 2 cells wherever a tile begins.  Each
+// lane counts and then writes the listed slots of one cell (one cell piece
+// after another per warp, 32 slots at a time, took 25-31 us, this form 14:
+// a frame block's 64 pieces are one chain of loads each).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_plist(PorArgs a) {
     pdl_wait();
     pdl_launch();
+    constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     const int n_pfb = a.ctl->n_pfb;
@@ -262,8 +260,8 @@ __global__ void __launch_bounds__(256) k_plist(PorArgs a) {
             n0 = atomicAdd(&a.ctl->n_near, c);
             t0 = atomicAdd(&a.ctl->n_ptiles, nt);
         }
-        n0 = __shfl_sync(0xffffffffu, n0, 0);
-        t0 = __shfl_sync(0xffffffffu, t0, 0);
+        n0 = __shfl_sync(kAll, n0, 0);
+        t0 = __shfl_sync(kAll, t0, 0);
         const int inst = fb / a.nfb_local;
         const int l = fb - inst * a.nfb_local;
         const int fz = l % a.nf[2], fy = (l / a.nf[2]) % a.nf[1], fx = l / (a.nf[2] * a.nf[1]);
@@ -271,23 +269,34 @@ __global__ void __launch_bounds__(256) k_plist(PorArgs a) {
         frame_cells(a, 0, fx, x0, x1);
         frame_cells(a, 1, fy, y0, y1);
         frame_cells(a, 2, fz, z0, z1);
+        const int npy = (y1 - y0) / 2 + 1, nz = z1 - z0 + 1, pieces = ((x1 - x0) / 2 + 1) * npy * nz * 4;
         int pos = n0;
-        // 2 x 2 x 2-cell sub-blocks in turn, so that consecutive tiles are compact
-        for (int bx = x0; bx <= x1; bx += 2)
-            for (int by = y0; by <= y1; by += 2)
-                for (int bz = z0; bz <= z1; bz += 2)
-                    for (int cx = bx; cx <= min(bx + 1, x1); ++cx)
-                        for (int cy = by; cy <= min(by + 1, y1); ++cy) {
-                            const int base = inst * a.gs.ncl + (cx * a.gs.dim[1] + cy) * a.gs.dim[2];
-                            const int s = a.gs.start[base + bz], e = a.gs.start[base + min(bz + 1, z1) + 1];
-                            for (int k0 = s; k0 < e; k0 += 32) {
-                                const int k = k0 + lane;
-                                const bool near = k < e && a.flag[k] != 0;
-                                const unsigned m = __ballot_sync(0xffffffffu, near);
-                                if (near) a.near_list[pos + __popc(m & ((1u << lane) - 1u))] = k;
-                                pos += __popc(m);
-                            }
-                        }
+        for (int p0 = 0; p0 < pieces; p0 += 32) {
+            const int p = p0 + lane, q = p >> 2, pencil = q / nz;
+            const int px = pencil / npy, py = (px & 1) ? npy - 1 - pencil % npy : pencil % npy;
+            const int cx = x0 + 2 * px + ((p >> 1) & 1), cy = y0 + 2 * py + (p & 1);
+            const int cz = (pencil & 1) ? z1 - q % nz : z0 + q % nz;
+            int s = 0, e = 0;
+            if (p < pieces && cx <= x1 && cy <= y1) {
+                const int base = inst * a.gs.ncl + (cx * a.gs.dim[1] + cy) * a.gs.dim[2] + cz;
+                s = a.gs.start[base];
+                e = a.gs.start[base + 1];
+            }
+            int count = 0;
+#pragma unroll 8
+            for (int k = s; k < e; ++k) count += a.flag[k] != 0;
+            int end = count;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(kAll, end, o);
+                if (lane >= o) end += v;
+            }
+            int to = pos + end - count;
+            pos += __shfl_sync(kAll, end, 31);
+            if (count > 0)
+                for (int k = s; k < e; ++k)
+                    if (a.flag[k] != 0) a.near_list[to++] = k;
+        }
         for (int t = lane; t < nt; t += 32) a.tiles[t0 + t] = make_int4(n0 + kPM * t, min(kPM, c - kPM * t), fb, 0);
     }
 }
@@ -295,11 +304,19 @@ __global__ void __launch_bounds__(256) k_plist(PorArgs a) {
 // ---------------------------------------------------------------------------
 // the normaliser on the tensor cores
 // ---------------------------------------------------------------------------
+// Bounded wait; on a timeout, or when another warp has given up, the CTA's abort
+// flag is set and false returned.
 __device__ __forceinline__ bool bwait(uint64_t* bar, uint32_t parity, PorSmem& sh, sphdem_ctl_t* ctl) {
-    if (mbar_wait(bar, parity, kPPolls)) return true;
-    sh.abort_flag = 1;
-    flag(ctl, SPHDEM_FLAG_TIMEOUT);
+    if (*(volatile int*)&sh.abort_flag == 0) {
+        if (mbar_wait(bar, parity, kPPolls)) return true;
+        sh.abort_flag = 1;
+        flag(ctl, SPHDEM_FLAG_TIMEOUT);
+    }
     return false;
+}
+// The same for a whole warp: every lane returns the same.
+__device__ __forceinline__ bool bwait_warp(uint64_t* bar, uint32_t parity, PorSmem& sh, sphdem_ctl_t* ctl) {
+    return __all_sync(0xffffffffu, bwait(bar, parity, sh, ctl));
 }
 
 // 16 columns of this thread's TMEM lane, loaded and waited for in one statement.
@@ -431,7 +448,17 @@ __global__ void __launch_bounds__(kPThreads, 2) k_porosity_mma(PorArgs a) {
     const Geo& G = a.gs;
     const int n_units = a.ctl->n_ptiles * kPSlabs;
     constexpr uint32_t idesc = umma::idesc_bf16(kPM, kPN);
-    uint32_t g = 0;          // chunks run so far by this CTA (same count in every role)
+    // chunks run so far by this CTA, the same in every role: candidate stage and
+    // its phase, accumulator and its phase
+    uint32_t stage = 0, sphase = 0, buf = 0, bphase = 0;
+    auto next_chunk = [&]() {
+        if (++stage == kPStages) {
+            stage = 0;
+            sphase ^= 1u;
+        }
+        buf ^= 1u;
+        bphase ^= buf ^ 1u;
+    };
     bool issued = false;     // this CTA issued MMAs (drained before freeing TMEM)
 
     for (;;) {
@@ -474,9 +501,7 @@ __global__ void __launch_bounds__(kPThreads, 2) k_porosity_mma(PorArgs a) {
                 lo[1] = hi[1] = x.y;
                 lo[2] = hi[2] = x.z;
             }
-            float v[24];
-            subject_row(px, py, pz, v);
-            store_row(sh.A, tid, v);
+            make_row<true>(sh.A, tid, px, py, pz);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -572,16 +597,19 @@ __global__ void __launch_bounds__(kPThreads, 2) k_porosity_mma(PorArgs a) {
                 if (tid == 0) sh.cr[nchunks] = m - 1;
                 __syncthreads();
             }
-            if (warp >= kPMmaWarp + 1) {
-                // ---- staging: candidate rows and volumes ----
-                // thread st builds chunk positions st, st + 32 kPStageWarps, ...;
-                // the candidates of chunk c + 1 are loaded while chunk c's
-                // rows are built
-                const int st = tid - 32 * (kPMmaWarp + 1);
-                auto fetch = [&](int c, int t, float4& x) {
+            if (warp >= kPEpiWarps) {
+                // ---- staging: a candidate row and volume per thread; the next
+                // chunk's candidate is loaded while this one's row is built.
+                // Warp kPMmaWarp then issues the chunk's MMA (it waits for the
+                // accumulator there, at most two chunks ahead of the epilogue).
+                const int t = tid - 32 * kPEpiWarps;
+                // chunk position t (= slot offset mod 8 in its low bits) -> column:
+                // classes 0-3 fill columns 0-63, classes 4-7 columns 64-127
+                const int col = (t & 4) * 16 + (t >> 3) * 4 + (t & 3);
+                auto fetch = [&](int c) {
                     const int uu = c * kPN + t;
-                    x = make_float4(0.f, 0.f, 0.f, 0.f);  // V = 0: padding and past the end
-                    if (uu >= tot) return;
+                    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // V = 0: padding and past the end
+                    if (uu >= tot) return x;
                     int lo = crs ? sh.cr[c] : 0, hi = crs ? sh.cr[c + 1] : m - 1;
                     while (lo < hi) {
                         const int mid = (lo + hi + 1) >> 1;
@@ -592,72 +620,46 @@ __global__ void __launch_bounds__(kPThreads, 2) k_porosity_mma(PorArgs a) {
                     const int inf = sh.info[lo];
                     const int pf = inf & (kPAlign - 1), len = inf >> 3;
                     if (off2 >= pf && off2 < pf + len) x = __ldg(a.f_posv + sh.rs[lo] + off2);
+                    return x;
                 };
-                auto put = [&](int s, int t, const float4& x) {
-                    // chunk position t (= slot offset mod 8 in its low bits) -> column:
-                    // classes 0-3 fill columns 0-63, classes 4-7 columns 64-127
-                    const int col = (t & 4) * 16 + (t >> 3) * 4 + (t & 3);
-                    float v[24];
-                    candidate_row((x.x - cxw) * a.inv_h, (x.y - cyw) * a.inv_h, (x.z - czw) * a.inv_h, v);
-                    store_row(sh.B[s], col, v);
-                    sh.V[s][col] = x.w;
-                };
-                constexpr int kPerT = kPN / kPStageThreads;  // candidates per staging thread and chunk
-                float4 x[kPerT];
-                if (nchunks > 0)
-#pragma unroll
-                    for (int q = 0; q < kPerT; ++q) fetch(0, st + q * kPStageThreads, x[q]);
-                for (int c = 0; c < nchunks && !sh.abort_flag; ++c) {
-                    const uint32_t gi = g + c, s = gi % kPStages, k = gi / kPStages;
-                    if (k > 0 && !bwait(&sh.empty[s], (k - 1) & 1u, sh, a.ctl)) break;
-                    float4 y[kPerT];
-#pragma unroll
-                    for (int q = 0; q < kPerT; ++q) y[q] = x[q];
-                    if (c + 1 < nchunks)
-#pragma unroll
-                        for (int q = 0; q < kPerT; ++q) fetch(c + 1, st + q * kPStageThreads, x[q]);
-#pragma unroll
-                    for (int q = 0; q < kPerT; ++q) put(s, st + q * kPStageThreads, y[q]);
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (nchunks > 0) x = fetch(0);
+                for (int c = 0; c < nchunks; ++c) {
+                    if (!bwait_warp(&sh.empty[stage], sphase ^ 1u, sh, a.ctl)) break;
+                    const float4 y = x;
+                    if (c + 1 < nchunks) x = fetch(c + 1);
+                    make_row<false>(sh.B[stage], col, (y.x - cxw) * a.inv_h, (y.y - cyw) * a.inv_h,
+                                    (y.z - czw) * a.inv_h);
+                    sh.V[stage][col] = y.w;
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh.full[s]);  // one arrival per staging warp
-                }
-            } else if (warp == kPMmaWarp) {
-                // ---- MMA issue ----
-                if (lane == 0)
-                    for (int c = 0; c < nchunks && !sh.abort_flag; ++c) {
-                        const uint32_t gi = g + c, s = gi % kPStages, k = gi / kPStages;
-                        const uint32_t b = gi & 1u, kb = gi >> 1;
-                        if (!bwait(&sh.full[s], k & 1u, sh, a.ctl)) break;
-                        if (kb > 0 && !bwait(&sh.aempty[b], (kb - 1) & 1u, sh, a.ctl)) break;
-                        umma::fence_after();
-                        umma::mma_tile(tmem + b * kPN, sh.A, sh.B[s], kPK, idesc, false);
-                        umma::commit(&sh.afull[b]);
-                        umma::commit(&sh.empty[s]);
-                        issued = true;
+                    if (lane == 0) mbar_arrive(&sh.full[stage]);  // one arrival per staging warp
+                    if (warp == kPMmaWarp) {
+                        if (lane == 0 && bwait(&sh.full[stage], sphase, sh, a.ctl) &&
+                            bwait(&sh.aempty[buf], bphase ^ 1u, sh, a.ctl)) {
+                            umma::fence_after();
+                            umma::mma_tile(tmem + buf * kPN, sh.A, sh.B[stage], kPK, idesc, false);
+                            umma::commit(&sh.afull[buf]);
+                            umma::commit(&sh.empty[stage]);
+                            issued = true;
+                        }
+                        __syncwarp();
                     }
-                __syncwarp();
+                    next_chunk();
+                }
             } else {
                 // ---- epilogue: w(s) and the volume-weighted sums ----
-                for (int c = 0; c < nchunks && !sh.abort_flag; ++c) {
-                    const uint32_t gi = g + c, s = gi % kPStages, b = gi & 1u, kb = gi >> 1;
-                    const bool ok = mbar_wait(&sh.afull[b], kb & 1u, kPPolls);
-                    if (__any_sync(0xffffffffu, !ok)) {
-                        if (lane == 0) {
-                            sh.abort_flag = 1;
-                            flag(a.ctl, SPHDEM_FLAG_TIMEOUT);
-                        }
-                        break;
-                    }
+                for (int c = 0; c < nchunks; ++c) {
+                    if (!bwait_warp(&sh.afull[buf], bphase, sh, a.ctl)) break;
                     umma::fence_after();
-                    // this warp's half of the chunk, 32 columns per load; the
-                    // other epilogue warps of the sub-partition hide each load
+                    // this warp's half of the chunk, 16 columns per step, the
+                    // load of the next 16 behind the arithmetic; the other
+                    // epilogue warps of the sub-partition hide the first load
                     const int h0 = (warp >> 2) * (kPN / 2);
-                    const uint32_t tcol = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + b * kPN + h0;
+                    const uint32_t tcol = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + buf * kPN + h0;
                     {
-                        // 16 columns per step, the load of the next 16 behind the arithmetic
                         const Kpk K{pk2(0.125f), pk2(-0.9375f), pk2(2.5f), pk2(-2.5f), pk2(1.0f)};
-                        const uint32_t va = (uint32_t)__cvta_generic_to_shared(&sh.V[s][h0]);
+                        const uint32_t va = (uint32_t)__cvta_generic_to_shared(&sh.V[stage][h0]);
                         unsigned long long u01, u23;
                         memcpy(&u01, &acc01, 8);
                         memcpy(&u23, &acc23, 8);
@@ -673,12 +675,12 @@ __global__ void __launch_bounds__(kPThreads, 2) k_porosity_mma(PorArgs a) {
                     umma::fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        mbar_arrive(&sh.aempty[b]);
-                        mbar_arrive(&sh.empty[s]);
+                        mbar_arrive(&sh.aempty[buf]);
+                        mbar_arrive(&sh.empty[stage]);
                     }
+                    next_chunk();
                 }
             }
-            g += nchunks;
             __syncthreads();
         }
         // classes 4-7 (warps 4-7) are added to classes 0-3 (warps 0-3) of the same subject
