@@ -174,14 +174,15 @@ __global__ void k_pack(const float* __restrict__ theta, uint16_t* __restrict__ p
 // node MLP layers: out = epi(A[M,K] * B[N,K]^T + bias)
 // ---------------------------------------------------------------------------
 // add (optional, K = 128): rows r < n_add of the A operand are A[r] + add[r]
-// (the residual h + s * sum_j f_ij (.) h_j, formed while staging the tile).
+// (the residual h + s * sum_j f_ij (.) h_j, formed while staging the tile);
+// with clear, add[r] is zero afterwards (for the next round's sums).
 // a_out (optional): the staged operand rows are stored there too.
 // EPI_F32: z_out (optional) receives the output as well.
 // list (optional): the layer runs on rows 0 .. n_direct - 1 and on the list[0]
 // rows list[1 ..] (in any order: rows are independent); M bounds both.
 template <int K, int N, int EPI, bool IMG>
-__global__ void __launch_bounds__(kRT * kT) k_rows(const uint16_t* __restrict__ A, int M, const float* __restrict__ add,
-                                             int n_add, const uint16_t* __restrict__ B,
+__global__ void __launch_bounds__(kRT * kT) k_rows(const uint16_t* __restrict__ A, int M, float* add, int n_add,
+                                             bool clear, const uint16_t* __restrict__ B,
                                              const float* __restrict__ bias, float* __restrict__ out_f32,
                                              uint16_t* __restrict__ out_bf, float* __restrict__ z_out,
                                              int32_t* status, const int* __restrict__ list, int n_direct,
@@ -241,8 +242,9 @@ __global__ void __launch_bounds__(kRT * kT) k_rows(const uint16_t* __restrict__ 
             uint4 v = make_uint4(0, 0, 0, 0);
             if (row < M) v = __ldg(reinterpret_cast<const uint4*>(A + (size_t)row * K) + q);
             if (plus) {
-                const float4 a0 = __ldg(reinterpret_cast<const float4*>(add + (size_t)row * K + 8 * q));
-                const float4 a1 = __ldg(reinterpret_cast<const float4*>(add + (size_t)row * K + 8 * q + 4));
+                float4* at = reinterpret_cast<float4*>(add + (size_t)row * K + 8 * q);
+                const float4 a0 = at[0], a1 = at[1];
+                if (clear) at[0] = at[1] = make_float4(0.f, 0.f, 0.f, 0.f);
                 v = make_uint4(pack2(bf((uint16_t)v.x) + a0.x, bf((uint16_t)(v.x >> 16)) + a0.y),
                                pack2(bf((uint16_t)v.y) + a0.z, bf((uint16_t)(v.y >> 16)) + a0.w),
                                pack2(bf((uint16_t)v.z) + a1.x, bf((uint16_t)(v.z >> 16)) + a1.y),
@@ -1259,7 +1261,7 @@ int smem_opt_in(Kern k, uint32_t bytes) {
 
 template <int K, int N, int EPI, bool IMG>
 int rows(const uint16_t* A, int M, const uint16_t* B, const float* bias, float* out_f32, uint16_t* out_bf,
-         float* z_out, int32_t* status, cudaStream_t st, const float* add = nullptr, int n_add = 0,
+         float* z_out, int32_t* status, cudaStream_t st, float* add = nullptr, int n_add = 0, bool clear = false,
          const int* list = nullptr, int n_direct = 0, int early = 0, uint16_t* a_out = nullptr) {
     if (M <= 0) return SPHDEM_OK;
     constexpr uint32_t bytes = N * K * 2 + kT * K * 2 + 4 * (N < 2 ? 2 : N) + 16 + 16;
@@ -1267,7 +1269,7 @@ int rows(const uint16_t* A, int M, const uint16_t* B, const float* bias, float* 
     if (rc) return rc;
     const int tiles = (M + kT - 1) / kT;
     const int grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
-    launch_pdl(k_rows<K, N, EPI, IMG>, grid, kRT * kT, bytes, st, A, M, add, n_add, B, bias, out_f32, out_bf, z_out, status,
+    launch_pdl(k_rows<K, N, EPI, IMG>, grid, kRT * kT, bytes, st, A, M, add, n_add, clear, B, bias, out_f32, out_bf, z_out, status,
                list, n_direct, early, a_out);
     return launch_status("mpnn rows");
 }
@@ -1401,6 +1403,17 @@ extern "C" int sphdem_mpnn_graph(sphdem_grid_t* grid, const float* node_pos3, co
 
 namespace sd {
 namespace {
+// Before a forward pass: sender flags, the length of their list (if there is
+// one) and the aggregation sums of the first round.
+__global__ void k_clear(int* __restrict__ active, int n_nodes, int* __restrict__ list, float4* __restrict__ agg,
+                        long n_agg) {
+    pdl_wait();
+    pdl_launch();
+    const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x, stride = (long)gridDim.x * blockDim.x;
+    if (list && i0 == 0) list[0] = 0;
+    for (long i = i0; i < n_nodes; i += stride) active[i] = 0;
+    for (long i = i0; i < n_agg; i += stride) agg[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
 // Non-receiver senders of the current graph, each listed once: list[0] is
 // their count, list[1 ..] the nodes (order immaterial: node rows are
 // independent).  Edge count from the CSR offsets, bounded by the edge buffer
@@ -1428,19 +1441,16 @@ extern "C" int sphdem_mpnn_forward(const sphdem_mpnn_net_t* n, int store_pre, sp
     // node layers on the receivers and the other nodes that send (no other
     // node's rows are read, and none has a gradient)
     const int* list = nullptr;
-    if (n->active && n->active_list && nn > nr) {
-        cudaError_t e = zero_words(n->active, nn, st);
-        if (e == cudaSuccess) e = zero_words(n->active_list, 1, st);
-        if (e != cudaSuccess) {
-            set_error("mpnn_forward", e);
-            return SPHDEM_ERR_CUDA;
-        }
+    const bool listed = n->active && n->active_list && nn > nr;
+    launch_pdl(k_clear, 4 * sm_count(), 256, 0, st, n->active, listed ? nn : 0, listed ? n->active_list : nullptr,
+               reinterpret_cast<float4*>(n->agg), (long)nr * (kH / 4));
+    if (listed) {
         launch_pdl(k_mark_senders, 2 * sm_count(), 256, 0, st, n->offset, n->sender, nr, nn, n->edge_capacity,
                    n->active, n->active_list);
         list = n->active_list;
     }
     int rc = rows<16, 128, EPI_SILU, true>(n->x, nn, n->packed + P_N1, n->theta + SPHDEM_MPNN_N1_B, nullptr, n->h0,
-                                           store_pre ? n->z0 : nullptr, n->status, st, nullptr, 0, list, nr,
+                                           store_pre ? n->z0 : nullptr, n->status, st, nullptr, 0, false, list, nr,
                                            list != nullptr && !store_pre);
     if (rc) return rc;
     // Inference copies the weight images early: every kernel of the chain
@@ -1450,22 +1460,17 @@ extern "C" int sphdem_mpnn_forward(const sphdem_mpnn_net_t* n, int store_pre, sp
     a.early = !store_pre;
     const int eg = edge_grid(n, 1);
     for (int round = 0; round < 2; ++round) {
-        cudaError_t e = zero_words(n->agg, (long)nr * kH, st);
-        if (e != cudaSuccess) {
-            set_error("mpnn_forward", e);
-            return SPHDEM_ERR_CUDA;
-        }
         a.h = round == 0 ? n->h0 : n->h2;
         a.agg = n->agg;
         if (nr > 0 && (rc = edges<MODE_AGG>(a, eg, st))) return rc;
         if (round == 0)  // h1 = h0 + agg formed while staging (the backward pass reads it)
             if ((rc = rows<128, 128, EPI_SILU, true>(n->h0, nn, n->packed + P_N2, n->theta + SPHDEM_MPNN_N2_B, nullptr,
                                                      n->h2, store_pre ? n->z2 : nullptr, n->status, st, n->agg, nr,
-                                                     list, nr, !store_pre, store_pre ? n->h1 : nullptr)))
+                                                     true, list, nr, !store_pre, store_pre ? n->h1 : nullptr)))
                 return rc;
     }
     rc = rows<128, 16, EPI_F32, true>(n->h2, nr, n->packed + P_N3, n->theta + SPHDEM_MPNN_N3_B, n->out, nullptr, nullptr,
-                                      n->status, st, n->agg, nr, nullptr, 0, !store_pre, store_pre ? n->h3 : nullptr);
+                                      n->status, st, n->agg, nr, false, nullptr, 0, !store_pre, store_pre ? n->h3 : nullptr);
     if (rc) return rc;
     return launch_status("mpnn_forward");
 }
@@ -1521,7 +1526,7 @@ extern "C" int sphdem_mpnn_backward(const sphdem_mpnn_net_t* n, const sphdem_mpn
     add_segment(sums, take(ncta, 128 * 128), ncta, 128 * 128, 128 * 128, grad + SPHDEM_MPNN_N2_W);
     // first message round and the edge MLP: d_h0 = d_h1, + the scatter
     if ((rc = rows<128, 128, EPI_F32, true>(g->bf_a, nn, n->packed + P_N2T, nullptr, g->d_h1, nullptr, g->d_h0,
-                                            n->status, st, nullptr, 0, list, nr)))
+                                            n->status, st, nullptr, 0, false, list, nr)))
         return rc;
     a.g1 = g->d_h1;
     a.g2 = g->g2;
