@@ -9,12 +9,13 @@ from __future__ import annotations
 import ctypes as C
 from pathlib import Path
 
+import torch
+
 from .build import LIB
 
-c_float_p = C.POINTER(C.c_float)
-c_int_p = C.POINTER(C.c_int32)
-c_double_p = C.POINTER(C.c_double)
-c_u64_p = C.POINTER(C.c_uint64)
+# Pointer members are plain addresses: assigning an int costs a tenth of making
+# a typed pointer object (the step API sets up to 60 of them per call).
+c_float_p = c_int_p = c_double_p = c_u64_p = c_u16_p = C.c_void_p
 
 
 class SphT(C.Structure):
@@ -80,9 +81,6 @@ class CtxT(C.Structure):
                 ("ctl", C.c_void_p)]
 
 
-c_u16_p = C.POINTER(C.c_uint16)
-
-
 class MpnnNodesT(C.Structure):
     _fields_ = ([(n, c_float_p) for n in ("f_pos", "f_vel", "f_acc", "f_rho", "f_por")] + [("n_fluid", C.c_int32)]
                 + [(n, c_float_p) for n in ("d_pos", "d_vel", "d_acc", "d_rad")] + [("n_dem", C.c_int32)]
@@ -144,6 +142,7 @@ _SIGNATURES = {
     "sphdem_sphdem_onestep": ([C.c_void_p, C.c_void_p, C.c_int, C.c_void_p], C.c_int),
     "sphdem_run": ([C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p], C.c_int),
     "sphdem_release": ([C.c_void_p], C.c_int),
+    "sphdem_status_copy": ([C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p], C.c_int),
     "sphdem_graph_kernels": ([C.c_void_p, C.c_int], C.c_int),
     "sphdem_profile_step": ([C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p], C.c_int),
     "sphdem_shepard_sph": ([C.c_void_p, C.c_float, C.c_float, C.c_void_p], C.c_int),
@@ -252,13 +251,18 @@ def check(rc: int, what: str) -> None:
 
 
 def fptr(t):
-    """float* of a contiguous float32 tensor (or NULL for None)."""
-    return C.cast(t.data_ptr(), c_float_p) if t is not None else c_float_p()
+    """Address of a tensor's first element (None: NULL)."""
+    return t.data_ptr() if t is not None else None
 
 
-def iptr(t):
-    return C.cast(t.data_ptr(), c_int_p) if t is not None else c_int_p()
+iptr = dptr = fptr
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
-def dptr(t):
-    return C.cast(t.data_ptr(), c_double_p) if t is not None else c_double_p()
+def stream_of(device) -> int:
+    """Handle of torch's current CUDA stream on `device`."""
+    index = device.index
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(torch.cuda.current_device() if index is None else index)

@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import weakref
+from operator import attrgetter
 
 import torch
 
@@ -88,6 +89,10 @@ class StepContext:
         self.wall_key = None
         self.built = [False] * 4
         self._sig = None
+        self._grid_sig = [None] * 4
+        # every field of the four sets but the contact views, fetched in one call
+        self._fields = [attrgetter(*(n for n in s.field_names() if not n.startswith(("contact_", "tang_"))))
+                        for s in self.sets]
         self._status_host = torch.zeros(16, dtype=torch.int32, pin_memory=True)
         self._status_event = None
         # launch tuning (results do not depend on it): see autotune.py
@@ -187,13 +192,12 @@ class StepContext:
 
     # -- ctypes structure --------------------------------------------------------
     def _signature(self):
+        """Device addresses of every field: read afresh on each call, as a caller
+        may replace a field's tensor or its storage."""
         sig = []
-        for s in self.sets:
-            for name in s.field_names():
-                if name.startswith(("contact_", "tang_")):
-                    continue
-                sig.append(getattr(s, name).data_ptr())
-        return tuple(sig)
+        for get, s in zip(self._fields, self.sets):
+            sig += [t.data_ptr() for t in get(s)]
+        return sig
 
     def _fill(self) -> None:
         sig = self._signature()
@@ -244,8 +248,16 @@ class StepContext:
     def _fill_grids(self) -> None:
         lo, hi = self._domain()
         for k, (g, s) in enumerate(zip(self.grids, self.sets)):
-            g.ensure_geometry(lo, hi, s.n, self.device)
-            g.fill(getattr(self.ctx, ("grid_sph", "grid_bnd", "grid_dem", "grid_dembnd")[k]), s.n)
+            n = s.n
+            g.ensure_geometry(lo, hi, n, self.device)
+            # the grid's own box and buffers are replaced, never changed in place
+            inst = g.inst.data_ptr() if g.inst is not None else None
+            old = self._grid_sig[k]
+            if (old is not None and old[0] is g.geometry and old[1] is g.buffers and old[2] == g.ninst
+                    and old[3] == n and old[4] == inst):
+                continue
+            g.fill(getattr(self.ctx, ("grid_sph", "grid_bnd", "grid_dem", "grid_dembnd")[k]), n)
+            self._grid_sig[k] = (g.geometry, g.buffers, g.ninst, n, inst)
 
     def set_params(self, solv, scales=None) -> None:
         p = self.params
@@ -271,7 +283,7 @@ class StepContext:
 
     @property
     def stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _lib.stream_of(self.device)
 
     # -- grids -------------------------------------------------------------------
     def prepare(self, rebuild_moving=True, wall_key=None) -> None:
@@ -315,10 +327,15 @@ class StepContext:
             self._raise_for(int(self._status_host[3]))
 
     def post_status(self) -> None:
-        self._status_host.copy_(self.ctl, non_blocking=True)
-        if self._status_event is None:
+        st = self.stream
+        event = None
+        if self._status_event is not None:
+            event = self._status_event.cuda_event
+        _lib.check(self.lib.sphdem_status_copy(self.ctl.data_ptr(), self._status_host.data_ptr(), event, st),
+                   "status copy")
+        if event is None:  # torch makes the event's handle when it is first recorded
             self._status_event = torch.cuda.Event()
-        self._status_event.record()
+            self._status_event.record(torch.cuda.current_stream(self.device))
 
     def check_status(self) -> None:
         """Blocking check of the device status bits."""

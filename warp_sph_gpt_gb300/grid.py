@@ -124,7 +124,7 @@ class HashGrid:
         g.key = _lib.iptr(b["key"])
         g.cursor = _lib.iptr(b["cursor"])
         g.block_sums = _lib.iptr(b["block_sums"])
-        g.inst = _lib.iptr(self.inst) if self.inst is not None else _lib.c_int_p()
+        g.inst = _lib.iptr(self.inst)
 
     def sorted_order(self) -> torch.Tensor:
         """Slot -> point index of the last device build (for tests)."""

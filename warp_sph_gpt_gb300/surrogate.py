@@ -88,7 +88,7 @@ class Network:
         self.pack()
 
     def stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _lib.stream_of(self.device)
 
     def pack(self) -> None:
         _lib.check(self.lib.sphdem_mpnn_pack(_p(self.theta), _p(self.packed), self.stream()), "mpnn_pack")
@@ -132,8 +132,7 @@ class Network:
         return Network(cfg, device, theta=z["theta"])
 
 
-def _p(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p()
+_p = _lib.fptr  # address of a tensor's first element (None: NULL)
 
 
 @dataclass
@@ -159,6 +158,16 @@ class Sets:
         t = getattr(part, name) if src is None else src
         return t[a:b]
 
+    def address(self, which, name, src=None):
+        """Device address of view(which, name, src), without making the view."""
+        t = src if src is not None else getattr({"f": self.P, "d": self.D, "b": self.B, "w": self.W}[which], name)
+        r = getattr(self, which)
+        return t.data_ptr() if r is None else t.data_ptr() + min(r[0], t.shape[0]) * t.stride(0) * t.element_size()
+
+
+_NET_BUFFERS = ("node_pos4", "node_vel4", "x", "offset", "sender", "receiver", "z0", "h0", "agg", "h1", "z2", "h2",
+                "h3", "out", "active", "active_list")
+
 
 class Graph:
     """Device workspace of one radius graph and the network's activations."""
@@ -177,7 +186,7 @@ class Graph:
         self.scan = None
 
     def stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return _lib.stream_of(self.device)
 
     # -- buffers -------------------------------------------------------------------
     def _ensure(self, n_nodes: int, n_recv: int) -> None:
@@ -217,38 +226,28 @@ class Graph:
     def set_nodes(self, sets: Sets, acc=None) -> None:
         """Node inputs of the particle ranges in ``sets`` (fluid, DEM, wall, DEM wall)."""
         cfg = self.cfg
-        nf = sets.rng("f")[1] - sets.rng("f")[0]
-        nd = sets.rng("d")[1] - sets.rng("d")[0]
-        nb = sets.rng("b")[1] - sets.rng("b")[0]
-        nw = sets.rng("w")[1] - sets.rng("w")[0]
+        (f0, f1), (d0, d1), (b0, b1), (w0, w1) = (sets.rng(k) for k in "fdbw")
+        nf, nd, nb, nw = f1 - f0, d1 - d0, b1 - b0, w1 - w0
         self._ensure(nf + nd + nb + nw, nf + nd)
         self.n_nodes, self.n_recv = nf + nd + nb + nw, nf + nd
         self.n_fluid, self.n_dem = nf, nd
+        at = sets.address
         a = _lib.MpnnNodesT()
-        P, D = sets.P, sets.D
-        a.f_pos = _lib.fptr(sets.view("f", "pos"))
-        a.f_vel = _lib.fptr(sets.view("f", "vel"))
-        a.f_acc = _lib.fptr(sets.view("f", "acc", acc[0] if acc else None))
-        a.f_rho = _lib.fptr(sets.view("f", "rho"))
-        a.f_por = _lib.fptr(sets.view("f", "porosity"))
-        a.n_fluid = nf
-        a.d_pos = _lib.fptr(sets.view("d", "pos")) if nd else _lib.c_float_p()
-        a.d_vel = _lib.fptr(sets.view("d", "vel")) if nd else _lib.c_float_p()
-        a.d_acc = _lib.fptr(sets.view("d", "acc", acc[1] if acc else None)) if nd else _lib.c_float_p()
-        a.d_rad = _lib.fptr(sets.view("d", "radius")) if nd else _lib.c_float_p()
+        a.f_pos, a.f_vel, a.f_acc = at("f", "pos"), at("f", "vel"), at("f", "acc", acc[0] if acc else None)
+        a.f_rho, a.f_por, a.n_fluid = at("f", "rho"), at("f", "porosity"), nf
+        if nd:
+            a.d_pos, a.d_vel, a.d_acc = at("d", "pos"), at("d", "vel"), at("d", "acc", acc[1] if acc else None)
+            a.d_rad = at("d", "radius")
         a.n_dem = nd
-        a.b_pos = _lib.fptr(sets.view("b", "pos"))
-        a.b_rho = _lib.fptr(sets.view("b", "rho"))
-        a.n_wall = nb
-        a.w_pos = _lib.fptr(sets.view("w", "pos")) if nw else _lib.c_float_p()
-        a.w_rad = _lib.fptr(sets.view("w", "radius")) if nw else _lib.c_float_p()
+        a.b_pos, a.b_rho, a.n_wall = at("b", "pos"), at("b", "rho"), nb
+        if nw:
+            a.w_pos, a.w_rad = at("w", "pos"), at("w", "radius")
         a.n_dem_wall = nw
         a.rho0, a.inv_vscale, a.inv_ascale = cfg.rho0, 1.0 / cfg.v_scale, 1.0 / cfg.a_scale
         a.inv_radius = 1.0 / cfg.radius
         b = self.buf
-        a.node_pos3, a.node_pos4, a.node_vel4 = _lib.fptr(b["node_pos3"]), _lib.fptr(b["node_pos4"]), _lib.fptr(
-            b["node_vel4"])
-        a.x = C.cast(b["x"].data_ptr(), _lib.c_u16_p)
+        a.node_pos3, a.node_pos4, a.node_vel4 = _p(b["node_pos3"]), _p(b["node_pos4"]), _p(b["node_vel4"])
+        a.x = _p(b["x"])
         self.nodes = a
         _lib.check(self.lib.sphdem_mpnn_nodes(C.byref(a), self.stream()), "mpnn_nodes")
 
@@ -291,14 +290,10 @@ class Graph:
         n = _lib.MpnnNetT()
         n.n_nodes, n.n_recv, n.edge_capacity = self.n_nodes, self.n_recv, self.capacity
         n.inv_radius, n.inv_vscale, n.inv_norm = 1.0 / self.cfg.radius, 1.0 / self.cfg.v_scale, 1.0 / self.cfg.norm
-        u16 = lambda t: C.cast(t.data_ptr(), _lib.c_u16_p)
-        n.node_pos4, n.node_vel4, n.x = _lib.fptr(b["node_pos4"]), _lib.fptr(b["node_vel4"]), u16(b["x"])
-        n.offset, n.sender, n.receiver = _lib.iptr(b["offset"]), _lib.iptr(b["sender"]), _lib.iptr(b["receiver"])
-        n.theta, n.packed = _lib.fptr(net.theta), u16(net.packed)
-        n.z0, n.h0, n.agg, n.h1 = _lib.fptr(b["z0"]), u16(b["h0"]), _lib.fptr(b["agg"]), u16(b["h1"])
-        n.z2, n.h2, n.h3, n.out = _lib.fptr(b["z2"]), u16(b["h2"]), u16(b["h3"]), _lib.fptr(b["out"])
-        n.status = C.cast(self.ctl.data_ptr() + 12, _lib.c_int_p)
-        n.active, n.active_list = _lib.iptr(b["active"]), _lib.iptr(b["active_list"])
+        for k in _NET_BUFFERS:
+            setattr(n, k, b[k].data_ptr())
+        n.theta, n.packed = net.theta.data_ptr(), net.packed.data_ptr()
+        n.status = self.ctl.data_ptr() + 12
         return n
 
     def forward(self, net: Network, store_pre: bool = False) -> torch.Tensor:
@@ -319,12 +314,11 @@ class Graph:
                              bf_b=torch.zeros(r, 16, dtype=torch.int16, device=self.device),
                              partial=torch.zeros(int(self.lib.sphdem_mpnn_partial_floats()), **f32))
         gb = self.gbuf
-        u16 = lambda t: C.cast(t.data_ptr(), _lib.c_u16_p)
         g = _lib.MpnnGradT()
-        g.d_out = _lib.fptr(d_out if d_out is not None else self.buf["d_out"])
-        g.g2, g.d_h2, g.d_h1, g.d_h0 = (_lib.fptr(gb[k]) for k in ("g2", "d_h2", "d_h1", "d_h0"))
-        g.bf_a, g.bf_b = u16(gb["bf_a"]), u16(gb["bf_b"])
-        g.partial, g.grad = _lib.fptr(gb["partial"]), _lib.fptr(net.grad)
+        g.d_out = _p(d_out if d_out is not None else self.buf["d_out"])
+        for k in ("g2", "d_h2", "d_h1", "d_h0", "bf_a", "bf_b", "partial"):
+            setattr(g, k, gb[k].data_ptr())
+        g.grad = net.grad.data_ptr()
         netst = self._net(net)
         _lib.check(self.lib.sphdem_mpnn_backward(C.byref(netst), C.byref(g), self.stream()), "mpnn_backward")
         return net.grad
@@ -355,21 +349,21 @@ def _apply(lib, graph: Graph, sets: Sets, net_out, cfg: SurrogateConfig, target_
     """Prior + correction into the particle arrays, or (target_state given) the
     normalised residual target rows of the graph's receivers."""
     nf, nd = graph.n_fluid, graph.n_dem
-    f_pos, f_vel = sets.view("f", "pos"), sets.view("f", "vel")
-    f_acc = sets.view("f", "acc", acc[0] if acc else None)
-    d_pos = sets.view("d", "pos") if nd else None
-    d_vel = sets.view("d", "vel") if nd else None
-    d_acc = sets.view("d", "acc", acc[1] if acc else None) if nd else None
+    at = sets.address
+    f_pos, f_vel, f_acc = at("f", "pos"), at("f", "vel"), at("f", "acc", acc[0] if acc else None)
+    d_pos = d_vel = d_acc = None
+    if nd:
+        d_pos, d_vel, d_acc = at("d", "pos"), at("d", "vel"), at("d", "acc", acc[1] if acc else None)
     # host array read by the call itself (not by the kernel): a named local, so
     # it outlives the call whatever ctypes does with temporaries
     scale_host = (C.c_float * 4)(*(float(v) for v in cfg.scale))
     scale = C.c_void_p(C.addressof(scale_host))
     if target_state is None:
-        rc = lib.sphdem_mpnn_apply(_p(f_pos), _p(f_vel), _p(f_acc), nf, _p(d_pos), _p(d_vel), _p(d_acc), nd,
+        rc = lib.sphdem_mpnn_apply(f_pos, f_vel, f_acc, nf, d_pos, d_vel, d_acc, nd,
                                    _p(net_out), cfg.substeps, cfg.dt, scale, None, None, None, graph.stream())
     else:
         x_t, v_t = target_state
-        rc = lib.sphdem_mpnn_apply(_p(f_pos), _p(f_vel), _p(f_acc), nf, _p(d_pos), _p(d_vel), _p(d_acc), nd, None,
+        rc = lib.sphdem_mpnn_apply(f_pos, f_vel, f_acc, nf, d_pos, d_vel, d_acc, nd, None,
                                    cfg.substeps, cfg.dt, scale, _p(x_t), _p(v_t), _p(graph.buf["target"]),
                                    graph.stream())
     _lib.check(rc, "mpnn_apply")
