@@ -84,9 +84,6 @@ __device__ __forceinline__ uint16_t bf16_bits(float a) {
     return *reinterpret_cast<uint16_t*>(&h);
 }
 __device__ __forceinline__ float bf(uint16_t u) { return __uint_as_float((uint32_t)u << 16); }
-__device__ __forceinline__ void st_bf16(uint8_t* base, uint32_t off, float v) {
-    *reinterpret_cast<uint16_t*>(base + off) = bf16_bits(v);
-}
 
 __device__ __forceinline__ void raise_flag(int32_t* status, int bits) {
     if (status) atomicOr(status, bits);
@@ -352,10 +349,15 @@ constexpr uint32_t kImg128 = 128 * 128 * 2;  // 32 KB
 constexpr uint32_t EF_IMG1 = 0, EF_IMG2 = EF_IMG1 + kImg16, EF_B1 = EF_IMG2 + kImg128, EF_B2 = EF_B1 + 512,
                    EF_BARS = EF_B2 + 512, EF_SLOT = EF_BARS + 48, EF_PIPE = (EF_SLOT + 16 + 1023) / 1024 * 1024,
                    EF_P_XS = 0, EF_P_ZR = EF_P_XS + kImg16, EF_P_SR = EF_P_ZR + kImg128, EF_P_SJ = EF_P_SR + 512,
-                   EF_P_END = EF_P_SJ + 512, EF_P_H = EF_P_END + 16, EF_P_BYTES = EF_P_H + kImg128,
-                   EF_BYTES = EF_PIPE + 2 * EF_P_BYTES;
-static_assert(EF_PIPE % 1024 == 0 && EF_P_BYTES % 16 == 0 && EF_P_H % 16 == 0, "k_edges shared memory alignment");
-static_assert(EF_BYTES <= 227 * 1024, "k_edges shared memory");
+                   EF_P_END = EF_P_SJ + 512, EF_P_H = EF_P_END + 16;
+template <int MODE>
+struct EdgeSmem {
+    static constexpr uint32_t pipe = EF_P_H + (MODE == MODE_AGG ? kImg128 : 0u), bytes = EF_PIPE + 2 * pipe;
+    static constexpr int ctas = MODE == MODE_AGG ? 1 : 2;  // per SM
+};
+static_assert(EF_PIPE % 1024 == 0 && EF_P_H % 16 == 0, "k_edges shared memory alignment");
+static_assert(EdgeSmem<MODE_AGG>::bytes <= 227 * 1024 && 2 * (EdgeSmem<MODE_SCATTER>::bytes + 1024) <= 228 * 1024,
+              "k_edges shared memory");
 
 struct EdgeLoad {
     int r, j;
@@ -367,7 +369,7 @@ struct EdgeLoad {
 __device__ __forceinline__ void edge_load_ids(const EdgeArgs& a, int e, int E, EdgeLoad& L) {
     L.r = -1;
     L.j = -1;
-    if (e < E) {
+    if ((unsigned)e < (unsigned)E) {
         L.r = __ldg(a.receiver + e);
         L.j = __ldg(a.sender + e);
     }
@@ -397,9 +399,16 @@ __device__ __forceinline__ uint4 edge_pack(const EdgeArgs& a, const EdgeLoad& L)
 // TMEM columns [128 p, 128 p + 128): layer 1 lands there (lane = edge), is
 // consumed by its epilogue, and layer 2 (lane = feature) overwrites it.  In
 // both epilogues warps w and w + 4 of a pipeline read the same 32 TMEM lanes
-// and split the 128 columns.  The next tile's edge data are loaded while the
-// current tile's epilogue runs; the senders' latent rows are bulk-copied into
-// shared memory as soon as a tile's edges are known.
+// and split the 128 columns.  The next tile's edge features are built while
+// layer 1 runs and written once it has read the current ones.  Aggregation
+// bulk-copies the senders' latent rows into shared memory as soon as a tile's
+// edges are known, which leaves room for one CTA per SM; it is bound by the
+// waits between its MMAs and epilogues.  The scatter needs no rows, runs two
+// CTAs per SM and is bound by its 4-byte atomic adds (one per edge and
+// feature): 509k edges in 74 us, against 189 us with one CTA, the epilogue's
+// columns indexed at run time (in local memory) and a load of the receiver's g
+// waited for at each new receiver.  Aggregation without staged rows, two CTAs
+// per SM: no faster.
 constexpr int kPT = 256;  // threads per pipeline
 
 // Barrier of one 256-thread pipeline (named barrier 1 or 2, immediate ids).
@@ -433,7 +442,7 @@ __device__ __forceinline__ bool pipe_or256(bool v, int id) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
+__global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
     uint8_t* img1 = sm + EF_IMG1;
     uint8_t* img2 = sm + EF_IMG2;
@@ -444,7 +453,7 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
     const int wq = warp & 7, lanes = 32 * (wq & 3), half = wq >> 2;
     const int lt = plt & (kT - 1);  // TMEM lane of this thread
     const bool loader = plt < kT;
-    uint8_t* pb = sm + EF_PIPE + p * EF_P_BYTES;
+    uint8_t* pb = sm + EF_PIPE + p * EdgeSmem<MODE>::pipe;
     uint8_t* xs = pb + EF_P_XS;
     uint8_t* zr = pb + EF_P_ZR;
     int* sr = reinterpret_cast<int*>(pb + EF_P_SR);
@@ -482,19 +491,22 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
     constexpr uint32_t idesc = umma::idesc_bf16(128, 128);
     const int stride = 2 * gridDim.x;
     int tile = 2 * blockIdx.x + p;
-    EdgeLoad nxt;
+    EdgeLoad nxt;  // ids of the next tile; its particle state until it is packed
+    int r0 = -1, j0 = -1;
     nxt.r = nxt.j = -1;
     if (loader) {
         edge_load_ids(a, tile * kT + lt, E, nxt);
         edge_load_state(a, nxt);
+        r0 = nxt.r;
+        j0 = nxt.j;
+        *reinterpret_cast<uint4*>(xs + tile_off(lt, 0, 16)) = edge_pack(a, nxt);
+        *reinterpret_cast<uint4*>(xs + tile_off(lt, 8, 16)) = make_uint4(0, 0, 0, 0);
+        edge_load_ids(a, (tile + stride) * kT + lt, E, nxt);
     }
     for (; !failed && tile * kT < E; tile += stride) {
         if (loader) {
-            const EdgeLoad cur_e = nxt;
-            sr[lt] = cur_e.r;
-            sj[lt] = cur_e.j;
-            *reinterpret_cast<uint4*>(xs + tile_off(lt, 0, 16)) = edge_pack(a, cur_e);
-            *reinterpret_cast<uint4*>(xs + tile_off(lt, 8, 16)) = make_uint4(0, 0, 0, 0);
+            sr[lt] = r0;
+            sj[lt] = j0;
             if (MODE == MODE_AGG && lt == 0) {
                 const int valid = min(kT, E - tile * kT);
                 mbar_arrive_expect_tx(hbar, (uint32_t)valid * 256u);
@@ -517,8 +529,14 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
                 const bool flush = r >= 0 && (lt == kT - 1 || lt == kT / 2 - 1 || sr[lt + 1] != r);
                 const unsigned m = __ballot_sync(0xffffffffu, flush);
                 if ((lt & 31) == 0) reinterpret_cast<uint32_t*>(pb + EF_P_END)[lt >> 5] = m;
+            } else {
+                // first edges of the receivers' runs, and of each half-tile
+                const int r = sr[lt];
+                const bool start = r >= 0 && (lt == 0 || lt == kT / 2 || sr[lt - 1] != r);
+                const unsigned m = __ballot_sync(0xffffffffu, start);
+                if ((lt & 31) == 0) reinterpret_cast<uint32_t*>(pb + EF_P_END)[lt >> 5] = m;
             }
-            edge_load_ids(a, (tile + stride) * kT + lt, E, nxt);  // prefetch the next tile's ids
+            edge_load_state(a, nxt);  // the next tile's particle state
         }
         if (MODE == MODE_AGG) hpending = true;
         pending = true;
@@ -530,6 +548,12 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
             pending = false;
         }
         umma::fence_after();
+        if (loader && mine) {  // layer 1 has read its tile: the next one's edge features
+            *reinterpret_cast<uint4*>(xs + tile_off(lt, 0, 16)) = edge_pack(a, nxt);
+            r0 = nxt.r;
+            j0 = nxt.j;
+            edge_load_ids(a, (tile + 2 * stride) * kT + lt, E, nxt);
+        }
         // layer-1 epilogue: lane = edge, this half's 64 hidden units
 #pragma unroll
         for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {
@@ -554,7 +578,8 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
             umma::mma_tile(tmem, img2, zr, 128, idesc, false);  // D[c][e], over layer 1's columns
             umma::commit(bar);
         }
-        if (loader) edge_load_state(a, nxt);  // the next tile's particle state
+        float gnext = 0.0f;
+        if (MODE == MODE_SCATTER && sr[64 * half] >= 0) gnext = __ldg(a.g + (size_t)sr[64 * half] * kH + lt);
         pending = true;
         mine = mbar_wait(bar, phase, kPolls);
         if (mine) {
@@ -565,7 +590,6 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
         // layer-2 epilogue: lane = feature c, this half's 64 edges of the tile
         const int c = lt;
         const float bc = b2[c];
-        int cur = -1;
         float gval = 0.0f;
         if (MODE == MODE_AGG) {
             hmine = mbar_wait(hbar, hphase, kPolls);
@@ -604,19 +628,34 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
                 }
             }
         } else {
+            // Edges of one receiver follow each other: its g is read once, one
+            // run ahead of its use.
+            const uint32_t* first = reinterpret_cast<const uint32_t*>(pb + EF_P_END) + 2 * half;
+            const unsigned long long starts = first[0] | (unsigned long long)first[1] << 32;
+            const int valid = E - tile * kT - 64 * half;  // edges of this half-tile
+            float* dhc = a.dh + c;
 #pragma unroll 1
-            for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {
-                float v[32];
-                umma::tmem_ld32(umma::taddr(tmem, lanes, c0), v);
-#pragma unroll 4
-                for (int i = 0; i < 32; ++i) {
-                    const int rr = sr[c0 + i];
-                    if (rr < 0) continue;
-                    if (rr != cur) {
-                        cur = rr;
-                        gval = __ldg(a.g + (size_t)rr * kH + c) * a.inv_norm;
+            for (int w = 0; w < 64 && w < valid; w += 8) {
+                const int c0 = 64 * half + w;
+                int j[8];
+                *reinterpret_cast<int4*>(j) = *reinterpret_cast<const int4*>(sj + c0);
+                *reinterpret_cast<int4*>(j + 4) = *reinterpret_cast<const int4*>(sj + c0 + 4);
+                float v[8];
+                umma::tmem_ld8(umma::taddr(tmem, lanes, c0), v);
+                const uint32_t runs = (uint32_t)(starts >> w) & 0xffu;
+                if (runs == 0u && w + 8 <= valid) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) atomicAdd(dhc + (size_t)j[i] * kH, (v[i] + bc) * gval);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if (runs & (1u << i)) {
+                            gval = gnext * a.inv_norm;
+                            const unsigned long long later = starts >> (w + i) >> 1;
+                            if (later) gnext = __ldg(a.g + (size_t)sr[c0 + i + __ffsll(later)] * kH + c);
+                        }
+                        if (j[i] >= 0) atomicAdd(dhc + (size_t)j[i] * kH, (v[i] + bc) * gval);
                     }
-                    atomicAdd(a.dh + (size_t)sj[c0 + i] * kH + c, (v[i] + bc) * gval);
                 }
             }
         }
@@ -640,7 +679,8 @@ __global__ void __launch_bounds__(2 * kPT, 1) k_edges(EdgeArgs a) {
 // edge inputs by edges, W2 as the forward image.
 constexpr uint32_t EB_IMG1 = 0, EB_IMG2 = EB_IMG1 + kImg16, EB_XS = EB_IMG2 + kImg128, EB_ZR = EB_XS + kImg16,
                    EB_DFT = EB_ZR + kImg128, EB_B2 = EB_DFT + kImg128, EB_SR = EB_B2 + 512, EB_SJ = EB_SR + 512,
-                   EB_MASK = EB_SJ + 512, EB_BARS = EB_MASK + 2048, EB_SLOT = EB_BARS + 16, EB_BYTES = EB_SLOT + 16;
+                   EB_MASK = EB_SJ + 512, EB_START = EB_MASK + 2048, EB_BARS = EB_START + 16,
+                   EB_SLOT = EB_BARS + 16, EB_BYTES = EB_SLOT + 16;
 static_assert(2 * (EB_BYTES + 1024) <= 228 * 1024, "k_edges_bwd: two CTAs per SM");
 constexpr int kBT = 512;  // threads: warps w, w + 4, w + 8, w + 12 share 32 TMEM lanes and split the 128 columns
 
@@ -649,9 +689,10 @@ constexpr int kBT = 512;  // threads: warps w, w + 4, w + 8, w + 12 share 32 TME
 // dF^T Z, dZ = W2^T dF^T, dP = dZ relu', dW1 += dP^T X.  What bounds it is the
 // work between the MMAs (per edge and feature: the products, a 4-byte atomic
 // add, two roundings), so it takes 4 threads per TMEM lane and two CTAs per SM
-// that fill each other's waits.  One thread per lane, one CTA per SM and
-// transposed copies of Z, dF and X written element by element took 1,108 us
-// for 509k edges; this form takes 254 us.
+// that fill each other's waits, and reads eight senders' rows at a time and a
+// receiver's g one run of edges ahead.  One thread per lane, one CTA per SM
+// and transposed copies of Z, dF and X written element by element took 1,108
+// us for 509k edges, an edge at a time 254 us; this form takes 194 us.
 // TMEM columns: [0,128) layer 1, layer 2, dZ, then dW1 of the tile; [128,256) dW2.
 __global__ void __launch_bounds__(kBT, 2) k_edges_bwd(EdgeArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -664,6 +705,7 @@ __global__ void __launch_bounds__(kBT, 2) k_edges_bwd(EdgeArgs a) {
     int* sr = reinterpret_cast<int*>(sm + EB_SR);
     int* sj = reinterpret_cast<int*>(sm + EB_SJ);
     uint32_t* mask = reinterpret_cast<uint32_t*>(sm + EB_MASK);  // [hidden unit / 32][edge]: z > 0
+    uint32_t* start = reinterpret_cast<uint32_t*>(sm + EB_START);  // bit per edge: the first of its receiver's
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + EB_BARS);
     uint32_t* slot = reinterpret_cast<uint32_t*>(sm + EB_SLOT);
     const int tid = threadIdx.x, warp = tid >> 5, lanes = 32 * (warp & 3), c0 = 32 * (warp >> 2);
@@ -683,16 +725,18 @@ __global__ void __launch_bounds__(kBT, 2) k_edges_bwd(EdgeArgs a) {
     constexpr uint32_t id128 = umma::idesc_bf16(128, 128), id16 = umma::idesc_bf16(128, 16);
     float db1 = 0.0f, db2 = 0.0f, w1[4] = {0.f, 0.f, 0.f, 0.f};
     EdgeLoad nxt;
+    uint4 xin = make_uint4(0, 0, 0, 0);  // the next tile's edge features
     nxt.r = nxt.j = -1;
     if (tid < kT) {
         edge_load_ids(a, blockIdx.x * kT + tid, E, nxt);
         edge_load_state(a, nxt);
+        xin = edge_pack(a, nxt);
     }
     for (int tile = blockIdx.x; !failed && tile * kT < E; tile += gridDim.x) {
         if (tid < kT) {
             sr[tid] = nxt.r;
             sj[tid] = nxt.j;
-            *reinterpret_cast<uint4*>(xs + tile_off(tid, 0, 16)) = edge_pack(a, nxt);
+            *reinterpret_cast<uint4*>(xs + tile_off(tid, 0, 16)) = xin;
             *reinterpret_cast<uint4*>(xs + tile_off(tid, 8, 16)) = make_uint4(0, 0, 0, 0);
         }
         operands_ready();
@@ -701,7 +745,13 @@ __global__ void __launch_bounds__(kBT, 2) k_edges_bwd(EdgeArgs a) {
             umma::mma_tile(tmem, xs, img1, 16, id128, false);  // P[e][k]
             umma::commit(&bars[0]);
         }
-        if (tid < kT) edge_load_ids(a, (tile + gridDim.x) * kT + tid, E, nxt);
+        if (tid < kT) {
+            // first edges of the receivers' runs, and of each 32 edges
+            const int r = sr[tid];
+            const unsigned m = __ballot_sync(0xffffffffu, r >= 0 && ((tid & 31) == 0 || sr[tid - 1] != r));
+            if ((tid & 31) == 0) start[tid >> 5] = m;
+            edge_load_ids(a, (tile + gridDim.x) * kT + tid, E, nxt);
+        }
         pending = true;
         if (!mma_done(bars, phase, mine)) { failed = true; break; }
         pending = false;
@@ -725,38 +775,66 @@ __global__ void __launch_bounds__(kBT, 2) k_edges_bwd(EdgeArgs a) {
             umma::commit(&bars[0]);
         }
         if (tid < kT) edge_load_state(a, nxt);
+        float g1n = 0.0f, g2n = 0.0f;
+        if (sr[c0] >= 0) {
+            g1n = __ldg(a.g1 + (size_t)sr[c0] * kH + row);
+            g2n = __ldg(a.g2 + (size_t)sr[c0] * kH + row);
+        }
         pending = true;
         if (!mma_done(bars, phase, mine)) { failed = true; break; }
         pending = false;
+        if (tid < kT) xin = edge_pack(a, nxt);
         {  // lane = feature: dF row, scatter of dh0, db2
+            // Edges of one receiver follow each other: its g1, g2 are read
+            // once, one run ahead of their use.
             const float bc = b2[row];
-            float v[32];
-            umma::tmem_ld32(umma::taddr(tmem, lanes, c0), v);
-            int cur = -1;
+            const uint32_t sw = start[c0 >> 5];
+            const int valid = E - tile * kT - c0;
             float g1v = 0.0f, g2v = 0.0f;
+#pragma unroll 1
+            for (int g = 0; g < 32; g += 8) {
+                int jj[8];
+                *reinterpret_cast<int4*>(jj) = *reinterpret_cast<const int4*>(sj + c0 + g);
+                *reinterpret_cast<int4*>(jj + 4) = *reinterpret_cast<const int4*>(sj + c0 + g + 4);
+                uint16_t h0v[8], h2v[8];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const int rr = sr[c0 + i], jj = sj[c0 + i];
-                float df = 0.0f;
-                if (rr >= 0) {
-                    if (rr != cur) {
-                        cur = rr;
-                        g1v = __ldg(a.g1 + (size_t)rr * kH + row) * a.inv_norm;
-                        g2v = __ldg(a.g2 + (size_t)rr * kH + row) * a.inv_norm;
-                    }
-                    const float h0v = bf(__ldg(a.h0 + (size_t)jj * kH + row));
-                    const float h2v = bf(__ldg(a.h2 + (size_t)jj * kH + row));
-                    df = g1v * h0v + g2v * h2v;
-                    atomicAdd(a.dh0 + (size_t)jj * kH + row, (v[i] + bc) * g1v);
+                for (int i = 0; i < 8; ++i) {
+                    const size_t at = (size_t)max(jj[i], 0) * kH + row;
+                    h0v[i] = __ldg(a.h0 + at);
+                    h2v[i] = __ldg(a.h2 + at);
                 }
-                db2 += df;
-                v[i] = df;
-            }
+                float v[8];
+                umma::tmem_ld8(umma::taddr(tmem, lanes, c0 + g), v);
+                const uint32_t runs = (sw >> g) & 0xffu;
+                if (runs == 0u && g + 8 <= valid) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                *reinterpret_cast<uint4*>(dft + tile_off(row, c0 + 8 * q, 128)) =
-                    make_uint4(pack2(v[8 * q], v[8 * q + 1]), pack2(v[8 * q + 2], v[8 * q + 3]),
-                               pack2(v[8 * q + 4], v[8 * q + 5]), pack2(v[8 * q + 6], v[8 * q + 7]));
+                    for (int i = 0; i < 8; ++i) {
+                        atomicAdd(a.dh0 + (size_t)jj[i] * kH + row, (v[i] + bc) * g1v);
+                        v[i] = g1v * bf(h0v[i]) + g2v * bf(h2v[i]);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if (runs & (1u << i)) {
+                            g1v = g1n * a.inv_norm;
+                            g2v = g2n * a.inv_norm;
+                            const uint32_t later = sw >> (g + i) >> 1;
+                            if (later) {
+                                const size_t at = (size_t)sr[c0 + g + i + __ffs(later)] * kH + row;
+                                g1n = __ldg(a.g1 + at);
+                                g2n = __ldg(a.g2 + at);
+                            }
+                        }
+                        const bool on = g + i < valid;
+                        if (on) atomicAdd(a.dh0 + (size_t)jj[i] * kH + row, (v[i] + bc) * g1v);
+                        v[i] = on ? g1v * bf(h0v[i]) + g2v * bf(h2v[i]) : 0.0f;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) db2 += v[i];
+                *reinterpret_cast<uint4*>(dft + tile_off(row, c0 + g, 128)) =
+                    make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+            }
         }
         operands_ready();
         if (tid == 0) {
@@ -1330,9 +1408,9 @@ int edge_grid(const sphdem_mpnn_net_t* n, int per_sm) {
 
 template <int MODE>
 int edges(const EdgeArgs& a, int grid, cudaStream_t st) {
-    int rc = smem_opt_in(k_edges<MODE>, EF_BYTES);
+    int rc = smem_opt_in(k_edges<MODE>, EdgeSmem<MODE>::bytes);
     if (rc) return rc;
-    launch_pdl(k_edges<MODE>, grid, 2 * kPT, EF_BYTES, st, a);
+    launch_pdl(k_edges<MODE>, grid, 2 * kPT, EdgeSmem<MODE>::bytes, st, a);
     return launch_status("mpnn edges");
 }
 
@@ -1517,7 +1595,7 @@ extern "C" int sphdem_mpnn_backward(const sphdem_mpnn_net_t* n, const sphdem_mpn
     EdgeArgs a = edge_args(n);
     a.g = g->g2;
     a.dh = g->d_h2;
-    if (nr > 0 && (rc = edges<MODE_SCATTER>(a, edge_grid(n, 1), st))) return rc;
+    if (nr > 0 && (rc = edges<MODE_SCATTER>(a, edge_grid(n, EdgeSmem<MODE_SCATTER>::ctas), st))) return rc;
     // second node layer
     p = take(cg, 128);
     k_act_grad<<<cg, 256, 0, st>>>(g->d_h2, n->z2, nn, list, nr, g->bf_a, p);
