@@ -344,8 +344,8 @@ constexpr uint32_t kImg16 = 128 * 16 * 2;   // 4 KB
 constexpr uint32_t kImg128 = 128 * 128 * 2;  // 32 KB
 // k_edges shared memory: the weight images once, then per pipeline an edge
 // feature tile, the hidden-activation tile, receiver/sender ids and an mbarrier.
-// The forward pass also stages the senders' latent rows (128 x 256 B) by
-// bulk copies issued when the tile is loaded, so they land during the MMAs.
+// The forward pass also stages the senders' latent rows (128 x 256 B); their
+// copies are issued with layer 1 and land during it and its epilogue.
 constexpr uint32_t EF_IMG1 = 0, EF_IMG2 = EF_IMG1 + kImg16, EF_B1 = EF_IMG2 + kImg128, EF_B2 = EF_B1 + 512,
                    EF_BARS = EF_B2 + 512, EF_SLOT = EF_BARS + 48, EF_PIPE = (EF_SLOT + 16 + 1023) / 1024 * 1024,
                    EF_P_XS = 0, EF_P_ZR = EF_P_XS + kImg16, EF_P_SR = EF_P_ZR + kImg128, EF_P_SJ = EF_P_SR + 512,
@@ -401,9 +401,11 @@ __device__ __forceinline__ uint4 edge_pack(const EdgeArgs& a, const EdgeLoad& L)
 // both epilogues warps w and w + 4 of a pipeline read the same 32 TMEM lanes
 // and split the 128 columns.  The next tile's edge features are built while
 // layer 1 runs and written once it has read the current ones.  Aggregation
-// bulk-copies the senders' latent rows into shared memory as soon as a tile's
+// copies the senders' latent rows into shared memory as soon as a tile's
 // edges are known, which leaves room for one CTA per SM; it is bound by the
-// waits between its MMAs and epilogues.  The scatter needs no rows, runs two
+// waits between its MMAs and epilogues (509k edges: 62 us with 16-byte
+// asynchronous copies by all threads, 64 us with a 256-byte bulk copy per
+// edge and a barrier to wait on).  The scatter needs no rows, runs two
 // CTAs per SM and is bound by its 4-byte atomic adds (one per edge and
 // feature): 509k edges in 74 us, against 189 us with one CTA, the epilogue's
 // columns indexed at run time (in local memory) and a load of the receiver's g
@@ -447,7 +449,7 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
     uint8_t* img1 = sm + EF_IMG1;
     uint8_t* img2 = sm + EF_IMG2;
     float* b2 = reinterpret_cast<float*>(sm + EF_B2);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + EF_BARS);  // [0],[1] MMAs, [2] weights, [3],[4] sender rows
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + EF_BARS);  // [0],[1] MMAs, [2] weights
     uint32_t* slot = reinterpret_cast<uint32_t*>(sm + EF_SLOT);
     const int tid = threadIdx.x, warp = tid >> 5, p = warp >> 3, plt = tid & (kPT - 1);
     const int wq = warp & 7, lanes = 32 * (wq & 3), half = wq >> 2;
@@ -460,10 +462,9 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
     int* sj = reinterpret_cast<int*>(pb + EF_P_SJ);
     uint8_t* hs = pb + EF_P_H;  // [128 edges][128] BF16 sender rows
     uint64_t* bar = &bars[p];
-    uint64_t* hbar = &bars[3 + p];
     const int bid = 1 + p;
     if (tid == 0) {
-        for (int b = 0; b < 5; ++b) mbar_init(&bars[b], 1);
+        for (int b = 0; b < 3; ++b) mbar_init(&bars[b], 1);
         fence_mbar_init();
         if (a.early) {  // the weight images are fixed: copy them while the previous kernel drains
             mbar_arrive_expect_tx(&bars[2], kImg16 + kImg128);
@@ -486,8 +487,8 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
         tma_load_1d(img2, a.img_e2, kImg128, &bars[2]);
     }
     bool failed = __syncthreads_or(!mbar_wait(&bars[2], 0, kPolls));
-    bool mine = true, hmine = true, pending = false, hpending = false;
-    uint32_t phase = 0, hphase = 0;
+    bool mine = true, pending = false;
+    uint32_t phase = 0;
     constexpr uint32_t idesc = umma::idesc_bf16(128, 128);
     const int stride = 2 * gridDim.x;
     int tile = 2 * blockIdx.x + p;
@@ -507,10 +508,6 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
         if (loader) {
             sr[lt] = r0;
             sj[lt] = j0;
-            if (MODE == MODE_AGG && lt == 0) {
-                const int valid = min(kT, E - tile * kT);
-                mbar_arrive_expect_tx(hbar, (uint32_t)valid * 256u);
-            }
         }
         fence_proxy_async_smem();
         umma::fence_before();
@@ -522,7 +519,6 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
         }
         if (loader) {
             if (MODE == MODE_AGG) {
-                if (sj[lt] >= 0) tma_load_1d(hs + lt * 256, a.h + (size_t)sj[lt] * kH, 256, hbar);
                 // edges after which the running sum is flushed: the last edge of a
                 // receiver's run, and the last valid edge of each half-tile
                 const int r = sr[lt];
@@ -538,7 +534,18 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
             }
             edge_load_state(a, nxt);  // the next tile's particle state
         }
-        if (MODE == MODE_AGG) hpending = true;
+        if (MODE == MODE_AGG) {  // the senders' latent rows, 16 bytes a thread
+            const int l = plt & 15;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int e = 16 * i + (plt >> 4), j = sj[e];
+                if (j >= 0)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                     smem_u32(hs + e * 256 + 16 * l)),
+                                 "l"(a.h + (size_t)j * kH + 8 * l)
+                                 : "memory");
+            }
+        }
         pending = true;
         // A wait that gives up is reported at the pipeline's next barrier,
         // which then reduces the outcome (what is read meanwhile is discarded).
@@ -570,6 +577,7 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
                 *reinterpret_cast<uint4*>(zr + tile_off(lt, k, 128)) = w;
             }
         }
+        if (MODE == MODE_AGG) asm volatile("cp.async.wait_all;" ::: "memory");
         fence_proxy_async_smem();
         umma::fence_before();
         if (pipe_or256(!mine, bid)) { failed = true; break; }
@@ -592,11 +600,6 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
         const float bc = b2[c];
         float gval = 0.0f;
         if (MODE == MODE_AGG) {
-            hmine = mbar_wait(hbar, hphase, kPolls);
-            if (hmine) {
-                hphase ^= 1u;
-                hpending = false;
-            }
             const uint16_t* h16 = reinterpret_cast<const uint16_t*>(hs) + c;
             const uint32_t* ends = reinterpret_cast<const uint32_t*>(pb + EF_P_END);
             // Segmented sums over the receiver-sorted edges; a group of 8
@@ -660,11 +663,10 @@ __global__ void __launch_bounds__(2 * kPT, EdgeSmem<MODE>::ctas) k_edges(EdgeArg
             }
         }
         umma::fence_before();
-        if (pipe_or256(!mine || !hmine, bid)) { failed = true; break; }
+        if (pipe_or256(!mine, bid)) { failed = true; break; }
     }
     if (failed && plt == 0) raise_flag(a.status, SPHDEM_FLAG_TIMEOUT);
     if (pending && !mine) mbar_wait(bar, phase, kPolls);
-    if (MODE == MODE_AGG && hpending) mbar_wait(hbar, hphase, kPolls);  // copies still landing
     umma::fence_before();
     __syncthreads();
     if (warp == 0) {
