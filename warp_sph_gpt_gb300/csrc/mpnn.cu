@@ -389,7 +389,7 @@ __device__ __forceinline__ void edge_load_state(const EdgeArgs& a, EdgeLoad& L) 
 __device__ __forceinline__ uint4 edge_pack(const EdgeArgs& a, const EdgeLoad& L) {
     if (L.r < 0) return make_uint4(0, 0, 0, 0);
     const float dx = L.pj.x - L.pr.x, dy = L.pj.y - L.pr.y, dz = L.pj.z - L.pr.z;
-    const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
+    const float dist = sqrtf(fmaf(dz, dz, fmaf(dx, dx, __fmul_rn(dy, dy))));  // the same bits in every kernel
     return make_uint4(pack2(dx * a.inv_r, dy * a.inv_r), pack2(dz * a.inv_r, dist * a.inv_r),
                       pack2((L.vj.x - L.vr.x) * a.inv_vs, (L.vj.y - L.vr.y) * a.inv_vs),
                       pack2((L.vj.z - L.vr.z) * a.inv_vs, 1.0f));
