@@ -11,6 +11,8 @@
 
 namespace sd {
 
+constexpr uint32_t kPollNs = 2000;  // suspend-time hint of one poll
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -43,14 +45,19 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t
         : "memory");
 }
 
+// One poll.  The hint lets the hardware keep the warp suspended for up to 2 us
+// (it is woken when the phase completes); the default suspends for a small
+// part of that, and warps polling again and again took a tenth of the issue
+// slots of the porosity kernel: 2.73 -> 2.64 ms at 800k, 0.90 -> 0.86 at 100k
+// with submerged spheres.
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(kPollNs)
         : "memory");
     return ok != 0;
 }
