@@ -75,3 +75,35 @@ def test_sparse_and_scattered_particles(n):
     np.testing.assert_allclose(P.flt.cpu().numpy(), flt, rtol=2e-6, atol=1e-9)
     np.testing.assert_allclose(P.rho.cpu().numpy(), 1000.0, rtol=4e-6)
     assert torch.isfinite(P.acc).all()
+
+
+@pytest.mark.parametrize("n", [5000, 66000])
+@pytest.mark.parametrize("support", [0.03, 0.05])
+def test_sums_with_a_support_that_is_not_the_kernels(n, support):
+    """A support beyond 2 h, whose outer members weigh nothing, and one below,
+    which cuts the kernel off: several lanes (5,000) and one thread (66,000)."""
+    from scipy.spatial import cKDTree
+
+    from warp_sph_gpt_gb300 import HashGrid, kernels
+    from warp_sph_gpt_gb300.struct import BNDptl, SPHptl
+
+    h = 0.02
+    rng = np.random.default_rng(n)
+    P, B = SPHptl(n, "cuda"), BNDptl(7, "cuda")
+    side = (n / 60.0 * (4.0 / 3.0) * np.pi * (2.0 * h) ** 3) ** (1.0 / 3.0)  # ~60 neighbours
+    for part in (P, B):
+        part.pos.copy_(torch.tensor(rng.uniform(0.0, side, (part.n, 3)), dtype=torch.float32))
+        part.m.fill_(0.008)
+        part.rho.fill_(1000.0)
+    grids = [HashGrid(), HashGrid()]
+    for g, part in zip(grids, (P, B)):
+        g.build(part.pos, support)
+    kernels.Kernel_shepard_sph(P, B, *grids, support, h)
+    x = np.concatenate([P.pos.double().cpu().numpy(), B.pos.double().cpu().numpy()])
+    some = rng.choice(n, 300, replace=False)
+    want = np.empty(300)
+    for i, j in enumerate(cKDTree(x).query_ball_point(x[some], support)):
+        q = np.linalg.norm(x[j] - x[some[i]], axis=1) / h
+        want[i] = (0.008 / 1000.0 * 21.0 / (16.0 * np.pi * h ** 3) * np.maximum(1 - 0.5 * q, 0) ** 4 * (1 + 2 * q)).sum()
+    # ~120 additions and a dozen roundings a term of 2^-24, twice that for the FP32 positions
+    np.testing.assert_allclose(P.flt.cpu().numpy()[some], want, rtol=2e-5)

@@ -41,6 +41,34 @@ namespace {
 
 extern __shared__ __align__(16) unsigned char sph_smem[];
 
+// kern_w(k, fast_sqrt(d2)) of a finite d2, same bits: the guard of the root at
+// 0 and the end of the support are a maximum each.
+__device__ __forceinline__ float member_w(const Kern& k, float d2) {
+    const float q = (d2 * rsqrtf(fmaxf(d2, 1.0e-37f))) * k.inv_h;
+    const float u = fmaxf(1.0f - 0.5f * q, 0.0f);
+    const float u2 = u * u;
+    return k.cw * u2 * u2 * (1.0f + 2.0f * q);
+}
+
+// Squared distance to a candidate with d2_exact's rounding, x and y as an FP32
+// pair (a packed product is an FMA onto 0: the same rounding).
+struct Near2 {
+    unsigned long long nxy;
+    float z;
+    __device__ __forceinline__ explicit Near2(const float4& p) : z(p.z) {
+        asm("mov.b64 %0, {%1, %2};" : "=l"(nxy) : "f"(-p.x), "f"(-p.y));
+    }
+    __device__ __forceinline__ float d2(const float4& q) const {
+        float sx, sy;
+        asm("{\n\t.reg .b64 d;\n\tmov.b64 d, {%2, %3};\n\tadd.rn.ftz.f32x2 d, d, %4;\n\t"
+            "fma.rn.ftz.f32x2 d, d, d, %5;\n\tmov.b64 {%0, %1}, d;\n\t}"
+            : "=f"(sx), "=f"(sy)
+            : "f"(q.x), "f"(q.y), "l"(nxy), "l"(0ull));
+        const float dz = __fsub_rn(z, q.z);
+        return __fadd_rn(__fadd_rn(sx, sy), __fmul_rn(dz, dz));
+    }
+};
+
 // Subject of this thread and its lane among the subject's LANES.
 template <int LANES>
 __device__ __forceinline__ int subject_index(int& lane) {
@@ -49,22 +77,43 @@ __device__ __forceinline__ int subject_index(int& lane) {
     return (int)(t / LANES);
 }
 
-// body(ok, j, q, r) over the members (exact d2 < s2) of this lane's subject: a
+// body(ok, j, q, d2) over the members (exact d2 < s2) of this lane's subject: a
 // thread that walks every slot of the ball-trimmed ranges (LANES = 1), a warp
 // whose lanes stride through each range together (LANES = 32; its sums are
 // reduced across lanes at the end, a different, equally valid FP32 summation
 // order), or walk.cuh's walk.
-template <int LANES, class F>
+//
+// One thread per subject waits for its candidates more than it computes, so it
+// loads BATCH of them before it looks at the first.  Fluid density, 752k
+// particles: 585 us one at a time, 528 with 4, 510-520 with 6, 525 with 8; 100k,
+// nothing recorded: 97, 84, 80, 79.  The walls, most of which have no candidate
+// at all, take one at a time (178 us for 3.1M; 197 with 6).
+template <int LANES, int BATCH = 1, class F>
 __device__ __forceinline__ void visit_members(const Geo& g, const float4* __restrict__ posm, bool mine,
                                               const float4& p, float rq, float s2, int inst, int lane, F&& body) {
+    const Near2 near(p);
     auto one = [&](int j) {
         const float4 q = posm[j];
-        const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
-        if (r.d2 < s2) body(true, j, q, r);
+        const float d2 = near.d2(q);
+        if (d2 < s2) body(true, j, q, d2);
     };
-    if constexpr (LANES == 1) {
+    if constexpr (LANES == 1 && BATCH == 1) {
         for_each_range_ball(g, p.x, p.y, p.z, rq, inst, [&](int s, int e) {
             for (int j = s; j < e; ++j) one(j);
+        });
+    } else if constexpr (LANES == 1) {
+        for_each_range_ball(g, p.x, p.y, p.z, rq, inst, [&](int s, int e) {
+            for (int j = s; j < e; j += BATCH) {
+                float4 q[BATCH];
+#pragma unroll
+                for (int u = 0; u < BATCH; ++u)
+                    if (u == 0 || j + u < e) q[u] = posm[j + u];
+#pragma unroll
+                for (int u = 0; u < BATCH; ++u) {
+                    const float d2 = near.d2(q[u]);
+                    if ((u == 0 || j + u < e) && d2 < s2) body(true, j + u, q[u], d2);
+                }
+            }
         });
     } else if constexpr (LANES == 32) {
         warp_ranges_ball(g, p.x, p.y, p.z, rq, inst, [&](int s, int e) {
@@ -72,7 +121,8 @@ __device__ __forceinline__ void visit_members(const Geo& g, const float4* __rest
         });
     } else {
         WarpWalk<LANES>* walks = reinterpret_cast<WarpWalk<LANES>*>(sph_smem);
-        warp_walk<LANES>(g, posm, mine, p.x, p.y, p.z, rq, s2, inst, walks[threadIdx.x >> 5], body);
+        warp_walk<LANES>(g, posm, mine, p.x, p.y, p.z, rq, s2, inst, walks[threadIdx.x >> 5],
+                         [&](bool ok, int j, const float4& q, const D2& r) { body(ok, j, q, r.d2); });
     }
 }
 
@@ -82,7 +132,7 @@ __device__ __forceinline__ float lanes_sum(float v) {
 }
 
 // Thread-per-subject walk of the ball-trimmed ranges that records the walk mask
-// in rows: body(j, q, r) for the members; each range is taken in segments that
+// in rows: body(j, q, d2) for the members; each range is taken in segments that
 // end where a 32-bit mask word ends, the segment's member bits gathered in a
 // register and stored with the word.  Returns the slots walked.
 template <class Body>
@@ -101,7 +151,7 @@ __device__ __forceinline__ int walk_record(const Geo& g, const float4* __restric
                 const float4 q = posm[j];
                 const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
                 if (r.d2 < s2) {
-                    body(j, q, r);
+                    body(j, q, r.d2);
                     m |= bit;
                 }
             }
@@ -117,6 +167,9 @@ __device__ __forceinline__ int walk_record(const Geo& g, const float4* __restric
     if ((pos & 31) && (pos >> 5) < cap) rows[(size_t)(pos >> 5) * n + k] = (int32_t)word;
     return pos;
 }
+
+constexpr int kBatch = 6;       // candidates a thread of the density pass loads at a time
+constexpr int kNoRecord = -1;  // beside SPHDEM_NBR_SLOTS and SPHDEM_NBR_MASKS: no neighbour record kept
 
 struct DensArgs {
     Geo gs, gb;
@@ -138,7 +191,7 @@ struct DensArgs {
     float rho0, B, gamma;
 };
 
-template <int LANES, bool FLT, bool RHO, bool PRES>
+template <int LANES, bool FLT, bool RHO, bool PRES, int REC>
 __global__ void __launch_bounds__(256) k_density(DensArgs a) {
     pdl_wait();
     pdl_launch();
@@ -151,35 +204,35 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
     const int inst = mine ? inst_of(a.gs, o) : 0;
     float rho_sum = 0.0f, flt_sum = 0.0f;
     if ((LANES == 1 || LANES == 32) && !mine) return;
-    if (LANES == 1 && a.nbr != nullptr && a.fmt == SPHDEM_NBR_MASKS) {
+    if constexpr (LANES == 1 && REC == SPHDEM_NBR_MASKS) {
         int32_t* rows = a.nbr;
         const int wf = walk_record(a.gs, a.f_posm, p, a.rq, inst, a.s2, rows, n, k, a.cap,
-                                   [&](int j, const float4& q, const D2& r) {
-                                       const float w = kern_w(a.kern, fast_sqrt(r.d2));
+                                   [&](int j, const float4& q, float d2) {
+                                       const float w = member_w(a.kern, d2);
                                        if (RHO) rho_sum += q.w * w;
                                        if (FLT) flt_sum += a.f_vprev[j] * w;
                                    });
         int wb = 0;
         if (a.gb.ncl > 0)
             wb = walk_record(a.gb, a.b_posm, p, a.rq, inst, a.s2, rows + (size_t)a.cap * n, n, k, a.cap,
-                             [&](int j, const float4& q, const D2& r) {
-                                 const float w = kern_w(a.kern, fast_sqrt(r.d2));
+                             [&](int j, const float4& q, float d2) {
+                                 const float w = member_w(a.kern, d2);
                                  if (RHO) rho_sum += q.w * w;
                                  if (FLT) flt_sum += a.b_vprev[j] * w;
                              });
         rows[(size_t)(2 * a.cap) * n + k] = wf;
         rows[(size_t)(2 * a.cap + 1) * n + k] = wb;
     } else {
-        const bool list = LANES != 32 && a.nbr != nullptr;
+        constexpr bool list = LANES != 32 && REC == SPHDEM_NBR_SLOTS;
         const int shift = (threadIdx.x & 31) - lane;  // first lane of this subject
         // one kind's members: sums, and their slots into rows, up to the capacity
         auto kind = [&](const Geo& g, const float4* __restrict__ posm, const float* __restrict__ vprev, int first_row,
                         int count_row) {
             int found = 0;
-            visit_members<LANES>(g, posm, mine, p, a.rq, a.s2, inst, lane, [&](bool ok, int j, const float4& q,
-                                                                              const D2& r) {
+            visit_members<LANES, kBatch>(g, posm, mine, p, a.rq, a.s2, inst, lane, [&](bool ok, int j,
+                                                                                      const float4& q, float d2) {
                 if constexpr (LANES == 1 || LANES == 32) {
-                    const float w = kern_w(a.kern, fast_sqrt(r.d2));
+                    const float w = member_w(a.kern, d2);
                     if (RHO) rho_sum += q.w * w;
                     if (FLT) flt_sum += vprev[j] * w;
                     if (list) {
@@ -187,7 +240,7 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
                         ++found;
                     }
                 } else {
-                    const float w = ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f;
+                    const float w = ok ? member_w(a.kern, d2) : 0.0f;
                     if (list) {
                         const unsigned of = (__ballot_sync(0xffffffffu, ok) >> shift) & ((1u << (LANES & 31)) - 1u);
                         const int row = found + __popc(of & ((1u << lane) - 1u));
@@ -252,12 +305,12 @@ __global__ void __launch_bounds__(256) k_density_wall(WallArgs a) {
     float rho_sum = 0.0f;
     if (a.gs.ncl > 0)
         visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane,
-                             [&](bool ok, int j, const float4& q, const D2& r) {
+                             [&](bool ok, int j, const float4& q, float d2) {
                                  if constexpr (LANES == 1 || LANES == 32)
-                                     rho_sum += q.w * kern_w(a.kern, fast_sqrt(r.d2));
+                                     rho_sum += q.w * member_w(a.kern, d2);
                                  else
                                      rho_sum = ordered_fma<LANES>(rho_sum, ok ? q.w : 0.0f,
-                                                                  ok ? kern_w(a.kern, fast_sqrt(r.d2)) : 0.0f);
+                                                                  ok ? member_w(a.kern, d2) : 0.0f);
                              });
     rho_sum = lanes_sum<LANES>(rho_sum);
     if (lane != 0 || !mine) return;
@@ -510,7 +563,8 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
     // subjects without a record (none kept, or one that overflowed): the walk
     auto visit = [&](const Geo& g, const float4* __restrict__ posm, const float4* __restrict__ rp,
                      const float4* __restrict__ vel) {
-        auto member = [&](bool ok, int j, const float4& q, const D2& r) {
+        auto member = [&](bool ok, int j, const float4& q, float) {
+            const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
             ok = ok && r.d2 > kR2Min;
             Pair f = {};
             if (ok) f = force_pair<MODE>(a, r, vi, rpi.z, rpi.y, rpi.w, q, rp[j], vel[j]);
@@ -567,12 +621,12 @@ static int launch_block(int b) { return (b == 64 || b == 256) ? b : 128; }
 // Largest systems that take several lanes per subject; beyond them one thread
 // per subject fills the GPU and executes fewer instructions.  Measured (us, one
 // thread | several lanes):
-//   density (8 lanes)  12.5k: 114 | 34, 47k: 130 | 75, 752k: 580 | 897;
-//                      recording nothing, 100k: 95 | 119
+//   density (8 lanes)  12.5k: 66 | 30, 47k: 77 | 68, 100k: 102 | 123;
+//                      recording nothing, 100k: 79 | 119
 //   walls (4 lanes)    48k: 37 | 16, 118k: 40 | 21, 2.2M: 83 | 172
 //   force (4 lanes)    from records, 12.5k: 66 | 24, 47k: 67 | 47, 752k: 331 | 530;
 //                      by walks, 100k: 162 | 129
-constexpr int kDensityLanesMax = 128 * 1024, kDensityLanesMaxUnrecorded = 64 * 1024;
+constexpr int kDensityLanesMax = 64 * 1024;
 constexpr int kWallLanesMax = 256 * 1024;
 constexpr int kForceLanesMax = 128 * 1024;
 
@@ -585,21 +639,21 @@ static void loop_shape(int n, int& block, int& blocks, size_t& smem) {
     smem = LANES == 1 || LANES == 32 ? 0 : (size_t)(block / 32) * sizeof(WarpWalk<LANES == 32 ? 1 : LANES>);
 }
 
-template <int LANES>
+template <int LANES, int REC>
 static void launch_density(const DensArgs& a, bool flt, bool rho, bool pres, int bs, cudaStream_t st) {
     int nb;
     size_t smem;
     loop_shape<LANES>(a.n, bs, nb, smem);
     if (flt && rho && pres)
-        launch_pdl(k_density<LANES, true, true, true>, nb, bs, smem, st, a);
+        launch_pdl(k_density<LANES, true, true, true, REC>, nb, bs, smem, st, a);
     else if (!flt && rho && pres)
-        launch_pdl(k_density<LANES, false, true, true>, nb, bs, smem, st, a);
+        launch_pdl(k_density<LANES, false, true, true, REC>, nb, bs, smem, st, a);
     else if (flt && !rho)
-        launch_pdl(k_density<LANES, true, false, false>, nb, bs, smem, st, a);
+        launch_pdl(k_density<LANES, true, false, false, REC>, nb, bs, smem, st, a);
     else if (!flt && rho && !pres)
-        launch_pdl(k_density<LANES, false, true, false>, nb, bs, smem, st, a);
+        launch_pdl(k_density<LANES, false, true, false, REC>, nb, bs, smem, st, a);
     else
-        launch_pdl(k_density<LANES, true, true, false>, nb, bs, smem, st, a);
+        launch_pdl(k_density<LANES, true, true, false, REC>, nb, bs, smem, st, a);
 }
 
 template <int LANES>
@@ -657,11 +711,17 @@ int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool rh
     a.gamma = gamma;
     const int bs = launch_block(block);
     if (lanes == 32)
-        launch_density<32>(a, flt, rho, pres, bs, st);
-    else if ((a.nbr && a.fmt == SPHDEM_NBR_MASKS) || n > (a.nbr ? kDensityLanesMax : kDensityLanesMaxUnrecorded))
-        launch_density<1>(a, flt, rho, pres, bs, st);
+        launch_density<32, kNoRecord>(a, flt, rho, pres, bs, st);
+    else if (a.nbr && a.fmt == SPHDEM_NBR_MASKS)
+        launch_density<1, SPHDEM_NBR_MASKS>(a, flt, rho, pres, bs, st);
+    else if (a.nbr && n > kDensityLanesMax)
+        launch_density<1, SPHDEM_NBR_SLOTS>(a, flt, rho, pres, bs, st);
+    else if (a.nbr)
+        launch_density<8, SPHDEM_NBR_SLOTS>(a, flt, rho, pres, bs, st);
+    else if (n > kDensityLanesMax)
+        launch_density<1, kNoRecord>(a, flt, rho, pres, bs, st);
     else
-        launch_density<8>(a, flt, rho, pres, bs, st);
+        launch_density<8, kNoRecord>(a, flt, rho, pres, bs, st);
     return launch_status("density");
 }
 
