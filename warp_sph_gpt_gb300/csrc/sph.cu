@@ -303,7 +303,20 @@ __global__ void __launch_bounds__(256) k_density_wall(WallArgs a) {
     const float4 p = mine ? a.b_posm[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int inst = mine ? inst_of(a.gb, o) : 0;
     float rho_sum = 0.0f;
-    if (a.gs.ncl > 0)
+    // One thread a particle: most walls stand where there is no fluid, and a slab
+    // of whole columns (all y and z of the window at one x) without particles
+    // shows it in two loads.  3.1M walls of 64 dam breaks: 181 -> 149 us, 2.2M of
+    // one: 85 -> 52 (4 lanes a particle, which trim 32 columns at once: no gain).
+    bool wet = a.gs.ncl > 0;
+    if (LANES == 1 && wet) {
+        const Win w = window(a.gs, p.x, p.y, p.z, a.rq);
+        wet = false;
+        for (int cx = w.x0; cx <= w.x1; ++cx) {
+            const int* at = a.gs.start + inst * a.gs.ncl + (size_t)(cx * a.gs.dim[1]) * a.gs.dim[2];
+            wet |= __ldg(at + w.y0 * a.gs.dim[2]) != __ldg(at + (w.y1 + 1) * a.gs.dim[2]);
+        }
+    }
+    if (wet)
         visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane,
                              [&](bool ok, int j, const float4& q, float d2) {
                                  if constexpr (LANES == 1 || LANES == 32)
