@@ -256,7 +256,8 @@ typedef struct sphdem_params {
      * TMA bulk copies, single-instance grids; 2 = pair distances on the tensor
      * cores, uniform DEM h, needs the work.p* scratch), and the lanes per subject of
      * the density, wall-density and force loops (0/1 = one thread per
-     * particle; 32 = one warp per particle, for small systems). */
+     * particle or, for small systems, 4 or 8 lanes with the same bits; 32 = one
+     * warp per particle, another summation order). */
     int32_t block_sph;
     int32_t porosity_variant;
     int32_t lanes_sph;

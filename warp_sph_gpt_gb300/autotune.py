@@ -16,8 +16,8 @@ from pathlib import Path
 
 import torch
 
-# Fluid counts up to which one warp per particle is a candidate (beyond it one
-# thread per particle already fills the GPU).
+# Fluid counts up to which one warp per particle is a candidate beside one
+# thread or a few lanes (beyond it one thread per particle fills the GPU).
 WARP_LANES_MAX_FLUID = 200_000
 
 CACHE = Path(os.environ.get("SPHDEM_AUTOTUNE_CACHE", Path.home() / ".cache" / "warp_sph_gpt_gb300" / "autotune.json"))
