@@ -19,6 +19,7 @@
 // Sums use fixed lane/warp orders, so every result is deterministic.
 #include <cooperative_groups.h>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "demwalk.cuh"
 #include "tma.cuh"
@@ -463,6 +464,8 @@ constexpr int kIdSums = 9;  // flt, rho_f, vel_f xyz, pgf xyz, solid
 
 template <int CTAS>
 __global__ void __launch_bounds__(kIdThreads) k_interaction_dem(CplArgs a) {
+    static_assert(CTAS == 1 || CTAS == kIdRanks, "one rank per CTA of the cluster, or all in one CTA");
+    if (CTAS > 1) cluster_started();
     pdl_wait();
     pdl_launch();
     namespace cg = cooperative_groups;
@@ -527,6 +530,7 @@ __global__ void __launch_bounds__(kIdThreads) k_interaction_dem(CplArgs a) {
             if (lane == 0) red[wid][c] = v;
         }
         __syncthreads();
+        if (CTAS > 1) cluster_wait_started();  // the first CTA's shared memory is written next
         if (threadIdx.x < kIdSums) {
             float t = 0.0f;
             for (int k = 0; k < kIdThreads / 32; ++k) t += red[k][threadIdx.x];
