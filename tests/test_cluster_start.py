@@ -20,7 +20,7 @@ def _kernel_body(file, name):
     return text[head.end():at]
 
 
-@pytest.mark.parametrize("file,name", [("coupling.cu", "k_interaction_dem")])
+@pytest.mark.parametrize("file,name", [("coupling.cu", "k_interaction_dem"), ("mpnn.cu", "k_loss")])
 def test_peers_have_started_before_their_shared_memory_is_written(file, name):
     body = _kernel_body(file, name)
     first = body.index("map_shared_rank")

@@ -29,6 +29,7 @@
 #include <mutex>
 #include <utility>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "sphdem_mpnn.h"
 #include "umma.cuh"
@@ -1110,6 +1111,7 @@ __global__ void __cluster_dims__(kLossCtas, 1, 1) __launch_bounds__(1024)
            float* __restrict__ d_out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
+    cluster_started();
     __shared__ float red[32];
     __shared__ float sums[kLossCtas];
     const float inv = n > 0 ? 1.0f / (6.0f * (float)n) : 0.0f;
@@ -1126,6 +1128,7 @@ __global__ void __cluster_dims__(kLossCtas, 1, 1) __launch_bounds__(1024)
     s = warp_sum(s);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
+    cluster_wait_started();  // the first CTA's shared memory is written next
     if (threadIdx.x < 32) {
         const float t = warp_sum(red[threadIdx.x]);
         if (threadIdx.x == 0) cluster.map_shared_rank(sums, 0)[cluster.block_rank()] = t;
