@@ -386,6 +386,11 @@ int sphdem_prep_sphdem(sphdem_ctx_t* c, float support, float h, float sph_suppor
                        float sph_h, float eps_min, float eps_max, sphdem_stream_t s);   /* kernel/KERNEL_SPHDEM_interaction.py:43-115 */
 int sphdem_interaction_dem(sphdem_ctx_t* c, float mu, float eps_min, float eps_max,
                            float dt, sphdem_stream_t s);                                 /* kernel/KERNEL_SPHDEM_interaction.py:118-187 */
+/* The fluid grid only orders the work here: the particles are taken in its order
+ * if grid_sph.order is given and grid_sph.n is the particle count (it must then be
+ * built for these particles), else in point order, slower where neighbours in
+ * that order are apart.  The results are the same bits.  With several instances
+ * grid_sph.key is read as well. */
 int sphdem_interaction_sph(sphdem_ctx_t* c, float support, sphdem_stream_t s);         /* kernel/KERNEL_SPHDEM_interaction.py:190-226 */
 
 /* ---- point evaluations for known-answer tests -------------------------- */

@@ -573,8 +573,9 @@ __global__ void __launch_bounds__(kIdThreads) k_interaction_dem(CplArgs a) {
     st3(a.D.pressure_force, am, pf);
 }
 
-// Kernel_interaction_sph (+ Kernel_step_sph when INTEGRATE), grid order: the
-// particles of a warp share their spheres (demwalk.cuh).
+// Kernel_interaction_sph (+ Kernel_step_sph when INTEGRATE), grid order (point
+// order without a fluid grid): the particles of a warp share their spheres
+// (demwalk.cuh).
 constexpr int kReactThreads = 128;
 template <bool INTEGRATE>
 __global__ void __launch_bounds__(kReactThreads) k_react(CplArgs a) {
@@ -584,7 +585,7 @@ __global__ void __launch_bounds__(kReactThreads) k_react(CplArgs a) {
     DemTile& sh = tiles[threadIdx.x >> 5];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const bool mine = k < a.P.n;
-    const int i = mine ? a.gs.order[k] : 0;
+    const int i = mine ? (a.gs.order ? a.gs.order[k] : k) : 0;
     const float3 pi = mine ? ld3(a.P.pos, i) : make_float3(0.f, 0.f, 0.f);
     float3 fd = make_float3(0.f, 0.f, 0.f);
     if (a.D.n > 0)
@@ -723,6 +724,7 @@ int run_react(const sphdem_ctx_t* c, float support, float dt, bool integrate, cu
     if (n <= 0) return SPHDEM_OK;
     CplArgs a = make_args(c, support, 0.0f);
     a.dt = dt;
+    if (c->grid_sph.n != n) a.gs.order = nullptr;  // not a grid of these particles
     if (integrate)
         launch_pdl(k_react<true>, blocks_for(n, kReactThreads), kReactThreads, 0, st, a);
     else
