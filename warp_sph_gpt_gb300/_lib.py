@@ -142,6 +142,7 @@ _SIGNATURES = {
     "sphdem_sphdem_onestep": ([C.c_void_p, C.c_void_p, C.c_int, C.c_void_p], C.c_int),
     "sphdem_run": ([C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p], C.c_int),
     "sphdem_release": ([C.c_void_p], C.c_int),
+    "sphdem_status_copy": ([C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p], C.c_int),
     "sphdem_graph_kernels": ([C.c_void_p, C.c_int], C.c_int),
     "sphdem_profile_step": ([C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p], C.c_int),
     "sphdem_shepard_sph": ([C.c_void_p, C.c_float, C.c_float, C.c_void_p], C.c_int),

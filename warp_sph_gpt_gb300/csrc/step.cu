@@ -1098,6 +1098,21 @@ int sphdem_graph_kernels(sphdem_ctx_t* c, int variant) {
     return it->second.kernels[variant ? 1 : 0];
 }
 
+int sphdem_status_copy(const sphdem_ctl_t* ctl, int32_t* host, void* event, sphdem_stream_t stream) {
+    if (!ctl || !host) {
+        set_error_msg("status copy: null pointer");
+        return SPHDEM_ERR_INVALID;
+    }
+    static_assert(sizeof(sphdem_ctl_t) == 16 * sizeof(int32_t), "control words");
+    cudaError_t e = cudaMemcpyAsync(host, ctl, sizeof(*ctl), cudaMemcpyDeviceToHost, as_stream(stream));
+    if (e == cudaSuccess && event) e = cudaEventRecord((cudaEvent_t)event, as_stream(stream));
+    if (e != cudaSuccess) {
+        set_error("status copy", e);
+        return SPHDEM_ERR_CUDA;
+    }
+    return SPHDEM_OK;
+}
+
 int sphdem_release(sphdem_ctx_t* c) {
     std::lock_guard<std::mutex> lock(g_graph_mu);
     auto jt = g_jumps.find(c);

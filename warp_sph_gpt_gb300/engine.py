@@ -327,13 +327,15 @@ class StepContext:
             self._raise_for(int(self._status_host[3]))
 
     def post_status(self) -> None:
-        # torch's own copy: the pinned allocator then knows that the block is in
-        # use, and does not hand it out again before the copy has landed when
-        # this context is dropped meanwhile
-        self._status_host.copy_(self.ctl, non_blocking=True)
-        if self._status_event is None:
+        st = self.stream
+        event = None
+        if self._status_event is not None:
+            event = self._status_event.cuda_event
+        _lib.check(self.lib.sphdem_status_copy(self.ctl.data_ptr(), self._status_host.data_ptr(), event, st),
+                   "status copy")
+        if event is None:  # torch makes the event's handle when it is first recorded
             self._status_event = torch.cuda.Event()
-        self._status_event.record(torch.cuda.current_stream(self.device))
+            self._status_event.record(torch.cuda.current_stream(self.device))
 
     def check_status(self) -> None:
         """Blocking check of the device status bits."""
