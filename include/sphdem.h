@@ -36,7 +36,7 @@
 extern "C" {
 #endif
 
-#define SPHDEM_ABI_VERSION 11
+#define SPHDEM_ABI_VERSION 12
 
 /* work.nbr forms (params.nbr_format): int32 member slots, or walk masks. */
 #define SPHDEM_NBR_SLOTS 0
@@ -326,8 +326,9 @@ int sphdem_sphdem_onestep(sphdem_ctx_t* ctx, const sphdem_params_t* p, int step,
  * CUDA graph per context and replayed.  coupled=0 runs SPH_OneStep. */
 int sphdem_run(sphdem_ctx_t* ctx, const sphdem_params_t* p, int first_step,
                int n_steps, int coupled, sphdem_stream_t stream);
-/* Enqueues a copy of the 16 control words at ctl to host (pinned memory) and,
- * if event is not NULL, records that CUDA event behind it. */
+/* Enqueues a copy of the 16 control words at ctl to host (pinned memory, which
+ * must not be freed or used otherwise before the copy has landed) and, if event is
+ * not NULL, records that CUDA event behind it. */
 int sphdem_status_copy(const sphdem_ctl_t* ctl, int32_t* host, void* event, sphdem_stream_t stream);
 /* Releases the CUDA graph held for ctx (host-side object only). */
 int sphdem_release(sphdem_ctx_t* ctx);

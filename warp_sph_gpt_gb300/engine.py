@@ -8,6 +8,7 @@ host except the explicit status checks and the exact-length CSR views.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import math
 import weakref
@@ -71,6 +72,38 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
         raise RuntimeError(f"{name} must be a contiguous float32/int32 tensor")
 
 
+class _Posted:
+    """The pinned status words of one context and, per stream that copied to
+    them, an event behind its last copy.  The library enqueues the copies, so
+    torch's pinned allocator does not know of them: it would hand the block out
+    again while a copy is queued if it were freed with its context.  The words of
+    a dropped context therefore stay here until their events are done, looked
+    at whenever a context is made (a finaliser must not wait: it may run in the
+    middle of a capture)."""
+
+    dropped: collections.deque = collections.deque()
+
+    def __init__(self):
+        self.host = torch.zeros(16, dtype=torch.int32, pin_memory=True)
+        self.events = {}
+
+    def landed(self) -> bool:
+        try:
+            return all(ev.query() for ev in self.events.values())
+        except RuntimeError:  # recorded in a capture, whose graph may yet be launched
+            return False
+
+    @classmethod
+    def release_landed(cls) -> None:
+        for _ in range(len(cls.dropped)):
+            try:
+                p = cls.dropped.popleft()
+            except IndexError:  # another thread took it
+                return
+            if not p.landed():
+                cls.dropped.append(p)
+
+
 class StepContext:
     def __init__(self, sph, bnd, dem, dembnd, grids, device):
         self.device = torch.device(device)
@@ -93,8 +126,10 @@ class StepContext:
         # every field of the four sets but the contact views, fetched in one call
         self._fields = [attrgetter(*(n for n in s.field_names() if not n.startswith(("contact_", "tang_"))))
                         for s in self.sets]
-        self._status_host = torch.zeros(16, dtype=torch.int32, pin_memory=True)
-        self._status_event = None
+        _Posted.release_landed()
+        self._posted = _Posted()
+        self._status_host = self._posted.host
+        self._status_event = None  # behind the last copy
         # launch tuning (results do not depend on it): see autotune.py
         self.tuning = {"block_sph": 0, "porosity_variant": 2, "lanes_sph": 1, "nbr_cap": -1,
                        "nbr_format": _lib.NBR_SLOTS}
@@ -104,7 +139,7 @@ class StepContext:
         self._pkey = None
         self._alloc_work()
         addr = C.addressof(self.ctx)
-        weakref.finalize(self, _release, self.lib, addr)
+        weakref.finalize(self, _release, self.lib, addr, self._posted)
 
     # -- buffers ---------------------------------------------------------------
     def _alloc_work(self) -> None:
@@ -328,14 +363,13 @@ class StepContext:
 
     def post_status(self) -> None:
         st = self.stream
-        event = None
-        if self._status_event is not None:
-            event = self._status_event.cuda_event
-        _lib.check(self.lib.sphdem_status_copy(self.ctl.data_ptr(), self._status_host.data_ptr(), event, st),
-                   "status copy")
-        if event is None:  # torch makes the event's handle when it is first recorded
-            self._status_event = torch.cuda.Event()
-            self._status_event.record(torch.cuda.current_stream(self.device))
+        ev = self._posted.events.get(st)
+        _lib.check(self.lib.sphdem_status_copy(self.ctl.data_ptr(), self._status_host.data_ptr(),
+                                               ev.cuda_event if ev is not None else None, st), "status copy")
+        if ev is None:  # torch makes the event's handle when it is first recorded
+            ev = self._posted.events[st] = torch.cuda.Event()
+            ev.record(torch.cuda.current_stream(self.device))
+        self._status_event = ev
 
     def check_status(self) -> None:
         """Blocking check of the device status bits."""
@@ -354,7 +388,9 @@ class StepContext:
             raise FloatingPointError("non-finite particle position met while binning")
 
 
-def _release(lib, addr):
+def _release(lib, addr, posted):
+    if posted.events:
+        _Posted.dropped.append(posted)
     try:
         lib.sphdem_release(C.c_void_p(addr))
     except Exception:
