@@ -238,9 +238,11 @@ __device__ __forceinline__ void warp_ranges_ball(const Geo& g, float px, float p
 // by all lanes together, slot = -1 for lanes past the end, slots ascending over
 // the calls and lanes.  The lanes look up 32 columns at once and then take the
 // candidates of all of them in turn, so that a window of many short columns
-// (a few spheres each) costs one chain of loads per 32 candidates.
+// (a few spheres each) costs one chain of loads per 32 candidates.  With part /
+// parts, the warps that share one window take every parts-th 32 candidates each.
 template <class F>
-__device__ __forceinline__ void warp_candidates(const Geo& g, const Win& w, int inst, F&& f) {
+__device__ __forceinline__ void warp_candidates(const Geo& g, const Win& w, int inst, F&& f, int part = 0,
+                                                int parts = 1) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int ny = w.y1 - w.y0 + 1, ncols = w.x1 >= w.x0 && ny > 0 ? (w.x1 - w.x0 + 1) * ny : 0;
@@ -260,8 +262,8 @@ __device__ __forceinline__ void warp_candidates(const Geo& g, const Win& w, int 
         }
         const int total = __shfl_sync(kAll, end, 31);
         const unsigned some = __ballot_sync(kAll, n > 0);
-        for (int u0 = 0; u0 < total; u0 += 32) {
-            const int u = u0 + lane;
+        for (int q = part; 32 * q < total; q += parts) {
+            const int u = 32 * q + lane;
             int slot = -1;
             for (unsigned m = some; m; m &= m - 1) {
                 const int src = __ffs(m) - 1;
@@ -270,6 +272,7 @@ __device__ __forceinline__ void warp_candidates(const Geo& g, const Win& w, int 
             }
             f(slot);
         }
+        part = (part + parts - (total + 31) / 32 % parts) % parts;  // the next columns' turn
     }
 }
 

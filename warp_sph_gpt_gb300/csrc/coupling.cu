@@ -515,15 +515,21 @@ __global__ void __launch_bounds__(kIdThreads) k_interaction_dem(CplArgs a) {
                 }
             }
         }
-        // solid sum over DEM neighbours, a itself included (:165-168)
-        int chunk = 0;
-        warp_candidates(a.gd, window(a.gd, pa.x, pa.y, pa.z, rq), inst, [&](int slot) {
-            if (chunk++ % kIdWarps != me || slot < 0) return;
-            const int b = a.gd.order[slot];
-            const float3 pb = ld3(a.D.pos, b);
-            const D2 r = d2_exact(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
-            if (r.d2 < aux.z) s[8] += a.D.volume[b] * w_aux(aux, fast_sqrt(r.d2));
-        });
+        // solid sum over DEM neighbours, a itself included (:165-168).  A warp
+        // goes from its own 32 candidates to its next: 1,400 dry spheres, crowded,
+        // take 55 us (108 when every warp looked up all of them and left out the
+        // others'; 61 with one thread of the CTA for the whole sum), 3,000 in
+        // shallow water 251 (988; 595)
+        warp_candidates(
+            a.gd, window(a.gd, pa.x, pa.y, pa.z, rq), inst,
+            [&](int slot) {
+                if (slot < 0) return;
+                const int b = a.gd.order[slot];
+                const float3 pb = ld3(a.D.pos, b);
+                const D2 r = d2_exact(pa.x, pa.y, pa.z, pb.x, pb.y, pb.z);
+                if (r.d2 < aux.z) s[8] += a.D.volume[b] * w_aux(aux, fast_sqrt(r.d2));
+            },
+            me, kIdWarps);
 #pragma unroll
         for (int c = 0; c < kIdSums; ++c) {
             const float v = warp_sum(s[c]);
@@ -696,9 +702,10 @@ int run_interaction_dem(const sphdem_ctx_t* c, float mu, float eps_min, float ep
     a.eps_min = eps_min;
     a.eps_max = eps_max;
     a.dt = dt;
-    // a cluster per sphere while that leaves CTAs to spare: 2,000 spheres, most
-    // of them dry, took 339 us as clusters that each worked out all columns in
-    // every warp, and 168 as whole batches per warp
+    // a cluster per sphere, or one CTA (us): spheres in 100k particles, 160:
+    // 26 | 57, 512: 61 | 65, 1,000: 106 | 106, 1,400: 143 | 131; in 792k, 160:
+    // 72 | 182, 512: 184 | 188, 700: 237 | 211; in 12.5k, 160: 16 | 22, 512: 32 | 29,
+    // 800: 45 | 39; over 792k, most of them dry, 512: 55 | 121, 2,000: 92 | 126
     if (c->dem.n > kIdClusterMax) {
         launch_pdl(k_interaction_dem<1>, c->dem.n, kIdThreads, 0, st, a);
     } else {
