@@ -60,10 +60,19 @@ __device__ __forceinline__ void warp_dem_visit(const Geo& gd, bool mine, float p
                 sh.cell[lane] = make_int4(column / gd.dim[1], column % gd.dim[1], c % gd.dim[2], 0);
             }
             __syncwarp();
-            for (int i = 0; i < n; ++i) {
-                const float4 p = sh.p[i];
-                const D2 d = d2_exact(px, py, pz, p.x, p.y, p.z);
-                if (in && d.d2 < p.w && (!wide || in_window(o, sh.cell[i]))) body(i, d.d2);
+            if (!wide) {
+                for (int i = 0; i < n; ++i) {
+                    const float4 p = sh.p[i];
+                    const D2 d = d2_exact(px, py, pz, p.x, p.y, p.z);
+                    if (in && d.d2 < p.w) body(i, d.d2);
+                }
+            } else {
+                const Win own = window(gd, px, py, pz, rq);
+                for (int i = 0; i < n; ++i) {
+                    const float4 p = sh.p[i];
+                    const D2 d = d2_exact(px, py, pz, p.x, p.y, p.z);
+                    if (in && d.d2 < p.w && in_window(own, sh.cell[i])) body(i, d.d2);
+                }
             }
             __syncwarp();
         });
