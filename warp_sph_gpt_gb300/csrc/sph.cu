@@ -640,16 +640,18 @@ static float tait_B(float rho0, float c0, float gamma) { return rho0 * c0 * c0 /
 static int launch_block(int b) { return (b == 64 || b == 256) ? b : 128; }
 
 // Largest systems that take several lanes per subject; beyond them one thread
-// per subject fills the GPU and executes fewer instructions.  Measured (us, one
-// thread | several lanes):
-//   density (8 lanes)  12.5k: 66 | 30, 47k: 77 | 68, 100k: 102 | 123;
-//                      recording nothing, 100k: 79 | 119
-//   walls (4 lanes)    48k: 37 | 16, 118k: 40 | 21, 2.2M: 83 | 172
-//   force (4 lanes)    from records, 12.5k: 66 | 24, 47k: 67 | 47, 752k: 331 | 530;
-//                      by walks, 100k: 162 | 129
-constexpr int kDensityLanesMax = 64 * 1024;
-constexpr int kWallLanesMax = 256 * 1024;
-constexpr int kForceLanesMax = 128 * 1024;
+// per subject fills the GPU and executes fewer instructions.  Measured in steps of
+// tanks and of ensembles (us, several lanes | one thread):
+//   density (8 lanes)  8k: 28 | 72, 39k: 64 | 74, 49k: 71 | 79, 55k: 79 | 79, 64k: 89 | 82,
+//                      98k: 123 | 94; recording nothing, 39k: 59 | 67, 55k: 74 | 70
+//   walls (4 lanes)    48k: 15 | 39, 278k: 29 | 39, 387k: 47 | 49, 435k: 51 | 51,
+//                      450k: 47 | 51, 483k: 57 | 51, 773k: 92 | 64
+//   force (4 lanes)    from records, 8k: 21 | 49, 39k: 43 | 53, 55k: 51 | 53, 64k: 55 | 54,
+//                      98k: 79 | 62, 125k: 92 | 72;
+//                      by walks, 39k: 94 | 134, 80k: 125 | 151, 98k: 164 | 166, 123k: 202 | 179
+constexpr int kDensityLanesMax = 52 * 1024;
+constexpr int kWallLanesMax = 448 * 1024;
+constexpr int kForceLanesMax = 56 * 1024, kForceWalkLanesMax = 100 * 1024;
 
 // Blocks and shared memory of a loop with LANES lanes per subject (the walks
 // need 6-8 KB per warp: at most 128 threads, 48 KB without an opt-in).
@@ -807,7 +809,7 @@ int run_force(const sphdem_ctx_t* c, float support, float h, float mu, float g, 
     const int bs = launch_block(block);
     if (lanes == 32)
         launch_force<32>(a, mode, bs, st);
-    else if ((a.nbr && a.fmt == SPHDEM_NBR_MASKS) || n > kForceLanesMax)
+    else if ((a.nbr && a.fmt == SPHDEM_NBR_MASKS) || n > (a.nbr ? kForceLanesMax : kForceWalkLanesMax))
         launch_force<1>(a, mode, bs, st);
     else
         launch_force<4>(a, mode, bs, st);
