@@ -5,7 +5,8 @@ predicates and every sum has a fixed order -- only the speed does.  The
 autotuner times a few complete steps for each candidate (cell width factor of
 the fluid/wall grids, threads per block of the fluid loops, porosity
 implementation) on a fresh copy of the case, picks the fastest, and caches it
-in a small JSON file keyed by the case's sizes and the GPU name.
+in a small JSON file keyed by the case's sizes and the GPU name, beside the
+revision of the loops that it was timed with.
 """
 from __future__ import annotations
 
@@ -19,6 +20,10 @@ import torch
 # Fluid counts up to which one warp per particle is a candidate beside one
 # thread or a few lanes (beyond it one thread per particle fills the GPU).
 WARP_LANES_MAX_FLUID = 200_000
+
+# Revision of the loops that the options choose between, raised when one of them
+# becomes faster or slower: a choice stored under another revision is timed anew.
+LOOPS = 2
 
 CACHE = Path(os.environ.get("SPHDEM_AUTOTUNE_CACHE", Path.home() / ".cache" / "warp_sph_gpt_gb300" / "autotune.json"))
 
@@ -63,7 +68,7 @@ def autotune(make_case, key: str, ninst: int = 1, use_cache: bool = True, log=No
             cache = json.loads(path.read_text())
         except ValueError:
             cache = {}
-    if use_cache and key in cache:
+    if use_cache and cache.get(key, {}).get("loops") == LOOPS:
         return cache[key]
     table = []
     for cfg in candidates(ninst, n_fluid):
@@ -72,7 +77,7 @@ def autotune(make_case, key: str, ninst: int = 1, use_cache: bool = True, log=No
         if log:
             log(f"autotune {cfg}: {ms:.3f} ms/step")
     best = dict(min(table, key=lambda t: t[0])[1])
-    best["ms_per_step"] = min(t[0] for t in table)
+    best.update(ms_per_step=min(t[0] for t in table), loops=LOOPS)
     cache[key] = best
     if use_cache:
         path.parent.mkdir(parents=True, exist_ok=True)
