@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("streams", [1, 2])
 def test_a_late_status_copy_reaches_no_other_pinned_tensor(streams):
+    gc.collect()  # contexts of other tests
     s, P, B, D, W, grids = scene()
     ctx = context_for(P, B, D, W, tuple(grids))
     ctx.ctl[8:] = 77
