@@ -640,18 +640,27 @@ static float tait_B(float rho0, float c0, float gamma) { return rho0 * c0 * c0 /
 static int launch_block(int b) { return (b == 64 || b == 256) ? b : 128; }
 
 // Largest systems that take several lanes per subject; beyond them one thread
-// per subject fills the GPU and executes fewer instructions.  Measured in steps of
-// tanks and of ensembles (us, several lanes | one thread):
-//   density (8 lanes)  8k: 28 | 72, 39k: 64 | 74, 49k: 71 | 79, 55k: 79 | 79, 64k: 89 | 82,
-//                      98k: 123 | 94; recording nothing, 39k: 59 | 67, 55k: 74 | 70
-//   walls (4 lanes)    48k: 15 | 39, 278k: 29 | 39, 387k: 47 | 49, 435k: 51 | 51,
-//                      450k: 47 | 51, 483k: 57 | 51, 773k: 92 | 64
-//   force (4 lanes)    from records, 8k: 21 | 49, 39k: 43 | 53, 55k: 51 | 53, 64k: 55 | 54,
-//                      98k: 79 | 62, 125k: 92 | 72;
-//                      by walks, 39k: 94 | 134, 80k: 125 | 151, 98k: 164 | 166, 123k: 202 | 179
-constexpr int kDensityLanesMax = 52 * 1024;
-constexpr int kWallLanesMax = 448 * 1024;
-constexpr int kForceLanesMax = 56 * 1024, kForceWalkLanesMax = 100 * 1024;
+// per subject fills the GPU and executes fewer instructions.  The loops of a step
+// share the GPU with one another (the walls' with the density's, the porosity pass
+// with the force), and the shared memory of the several-lane walks is taken from
+// the others' L1, so the lines are drawn by whole steps, not by a loop's own time.
+// Step (us) with density, walls, force by one thread 000 ... by several lanes 111,
+// the form taken here marked *; SPH only, then coupled with spheres above the water:
+//   fluid  walls        000   001   010   011   111        000   001   010   011   111
+//    25k    118k        170   152   171   133   100*       164   137   188   149   113*
+//    49k    118k        181   172   197   156   145*       174   160   206   179   158*
+//    64k    180k        190   185   204   167   172*       175   171   212   193   191*
+//    96k    180k        245   238   261   217*  223        232   213   283   234*  246
+//   125k    278k        262   261*  283   245   278        246   245*  314   270   302
+//   150k    278k        267*  277   292   265   321        269*  279   323   295   351
+//   262k    450k        416*  439   485   432   536        409*  431   521   475   566
+// Ensembles: 55k / 242k 193 193 242 201 190*, 98k / 387k 235 245* 321 288 292,
+// 143k / 580k 293* 326 379 372 414.  Alone, 55k density 79 | 79 (lanes | one
+// thread), 435k walls 51 | 51, force from records 64k 55 | 54, 98k 79 | 62; by
+// walks (no records) 80k 125 | 151, 98k 164 | 166, 123k 202 | 179.
+constexpr int kDensityLanesMax = 64 * 1024;
+constexpr int kWallLanesMax = 256 * 1024;
+constexpr int kForceLanesMax = 128 * 1024, kForceWalkLanesMax = 100 * 1024;
 
 // Blocks and shared memory of a loop with LANES lanes per subject (the walks
 // need 6-8 KB per warp: at most 128 threads, 48 KB without an opt-in).
