@@ -671,21 +671,23 @@ static void loop_shape(int n, int& block, int& blocks, size_t& smem) {
     smem = LANES == 1 || LANES == 32 ? 0 : (size_t)(block / 32) * sizeof(WarpWalk<LANES == 32 ? 1 : LANES>);
 }
 
+// The steps' density, with the pressure and with or without records, and the
+// single kernels: the Shepard filter alone, the density alone.
 template <int LANES, int REC>
-static void launch_density(const DensArgs& a, bool flt, bool rho, bool pres, int bs, cudaStream_t st) {
+static void launch_density(const DensArgs& a, bool flt, bool pres, int bs, cudaStream_t st) {
     int nb;
     size_t smem;
     loop_shape<LANES>(a.n, bs, nb, smem);
-    if (flt && rho && pres)
+    if (flt && pres)
         launch_pdl(k_density<LANES, true, true, true, REC>, nb, bs, smem, st, a);
-    else if (!flt && rho && pres)
+    else if (pres)
         launch_pdl(k_density<LANES, false, true, true, REC>, nb, bs, smem, st, a);
-    else if (flt && !rho)
-        launch_pdl(k_density<LANES, true, false, false, REC>, nb, bs, smem, st, a);
-    else if (!flt && rho && !pres)
-        launch_pdl(k_density<LANES, false, true, false, REC>, nb, bs, smem, st, a);
-    else
-        launch_pdl(k_density<LANES, true, true, false, REC>, nb, bs, smem, st, a);
+    else if constexpr (REC == kNoRecord) {
+        if (flt)
+            launch_pdl(k_density<LANES, true, false, false, REC>, nb, bs, smem, st, a);
+        else
+            launch_pdl(k_density<LANES, false, true, false, REC>, nb, bs, smem, st, a);
+    }
 }
 
 template <int LANES>
@@ -714,8 +716,9 @@ static void launch_force(const ForceArgs& a, int mode, int bs, cudaStream_t st) 
         launch_pdl(k_force<LANES, 1>, nb, bs, smem, st, a);
 }
 
-int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool rho, bool pres, float rho0, float c0,
-                float gamma, cudaStream_t st, int block, int lanes, int nbr_cap, int nbr_format) {
+// flt with pres: the Shepard filter and the density; without: the filter alone.
+int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool pres, float rho0, float c0, float gamma,
+                cudaStream_t st, int block, int lanes, int nbr_cap, int nbr_format) {
     const int n = c->sph.n;
     if (n <= 0) return SPHDEM_OK;
     DensArgs a;
@@ -743,17 +746,17 @@ int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool rh
     a.gamma = gamma;
     const int bs = launch_block(block);
     if (lanes == 32)
-        launch_density<32, kNoRecord>(a, flt, rho, pres, bs, st);
+        launch_density<32, kNoRecord>(a, flt, pres, bs, st);
     else if (a.nbr && a.fmt == SPHDEM_NBR_MASKS)
-        launch_density<1, SPHDEM_NBR_MASKS>(a, flt, rho, pres, bs, st);
+        launch_density<1, SPHDEM_NBR_MASKS>(a, flt, pres, bs, st);
     else if (a.nbr && n > kDensityLanesMax)
-        launch_density<1, SPHDEM_NBR_SLOTS>(a, flt, rho, pres, bs, st);
+        launch_density<1, SPHDEM_NBR_SLOTS>(a, flt, pres, bs, st);
     else if (a.nbr)
-        launch_density<8, SPHDEM_NBR_SLOTS>(a, flt, rho, pres, bs, st);
+        launch_density<8, SPHDEM_NBR_SLOTS>(a, flt, pres, bs, st);
     else if (n > kDensityLanesMax)
-        launch_density<1, kNoRecord>(a, flt, rho, pres, bs, st);
+        launch_density<1, kNoRecord>(a, flt, pres, bs, st);
     else
-        launch_density<8, kNoRecord>(a, flt, rho, pres, bs, st);
+        launch_density<8, kNoRecord>(a, flt, pres, bs, st);
     return launch_status("density");
 }
 

@@ -27,8 +27,8 @@ int build_fluid(sphdem_ctx_t* c, cudaStream_t st);
 int gather_fluid(const sphdem_ctx_t* c, cudaStream_t st);
 int gather_wall(const sphdem_ctx_t* c, float support, float h, cudaStream_t st);
 int gather_wall_rho(const sphdem_ctx_t* c, cudaStream_t st);
-int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool rho, bool pres, float rho0, float c0,
-                float gamma, cudaStream_t st, int block = 0, int lanes = 1, int nbr_cap = 0, int nbr_format = 0);
+int run_density(const sphdem_ctx_t* c, float support, float h, bool flt, bool pres, float rho0, float c0, float gamma,
+                cudaStream_t st, int block = 0, int lanes = 1, int nbr_cap = 0, int nbr_format = 0);
 int run_density_wall(const sphdem_ctx_t* c, float support, float h, bool pres, float rho0, float c0, float gamma,
                      cudaStream_t st, int block = 0, int lanes = 1);
 int run_force(const sphdem_ctx_t* c, float support, float h, float mu, float g, int mode, cudaStream_t st,
@@ -93,7 +93,7 @@ bool shepard_due(const sphdem_params_t* p, int step) {
 int sph_part(sphdem_ctx_t* c, const sphdem_params_t* p, bool shep, bool write_pgf, cudaStream_t st) {
     if (shep) TRY(gather_wall_rho(c, st));
     const int cap = nbr_cap(c, p);
-    TRY(run_density(c, p->support, p->h, shep, true, true, p->rho0, p->c0, p->gamma, st, p->block_sph, p->lanes_sph,
+    TRY(run_density(c, p->support, p->h, shep, true, p->rho0, p->c0, p->gamma, st, p->block_sph, p->lanes_sph,
                     cap, p->nbr_format));
     TRY(run_density_wall(c, p->support, p->h, true, p->rho0, p->c0, p->gamma, st, p->block_sph, p->lanes_sph));
     sphdem_ctx_t cc = *c;
@@ -194,7 +194,7 @@ int coupled_onestep(sphdem_ctx_t* c, const sphdem_params_t* p, bool shep, cudaSt
     TRY(rec(f->wall, f->side3));
     const int cap = nbr_cap(c, p);
     if (!density_fresh)
-        TRY(run_density(c, p->support, p->h, shep, true, true, p->rho0, p->c0, p->gamma, st, p->block_sph,
+        TRY(run_density(c, p->support, p->h, shep, true, p->rho0, p->c0, p->gamma, st, p->block_sph,
                         p->lanes_sph, cap, p->nbr_format));
     TRY(rec(f->dens, st));
     // porosity branch.  One state: what needs positions only (the sorted
@@ -752,7 +752,7 @@ int jump_body(sphdem_ctx_t* c, const sphdem_params_t* p, const sphdem_jump_t* j,
     TRY(build_fluid(c, st));
     // the judge's density is the full density pass of the next plain step
     // (pressures, sorted copies, neighbour records), so that step can skip it
-    TRY(run_density(c, p->support, p->h, false, true, true, p->rho0, p->c0, p->gamma, st, p->block_sph, p->lanes_sph,
+    TRY(run_density(c, p->support, p->h, false, true, p->rho0, p->c0, p->gamma, st, p->block_sph, p->lanes_sph,
                     nbr_cap(c, p), p->nbr_format));
     const float* rho_old = j->keep + 6 * (size_t)c->sph.n + 6 * (size_t)c->dem.n;
     return sphdem_mpnn_maxdev(c->sph.rho, j->judge == 1 ? nullptr : rho_old, p->rho0, c->sph.n, 1.0f / p->rho0,
@@ -942,7 +942,7 @@ int capture_rollout(sphdem_ctx_t* c, const sphdem_params_t* p, const sphdem_jump
     if (!rc && !shepard_due(p, step + j->substeps + 1)) {
         rc = gather_fluid(c, cap);
         if (!rc)
-            rc = run_density(c, p->support, p->h, false, true, true, p->rho0, p->c0, p->gamma, cap, p->block_sph,
+            rc = run_density(c, p->support, p->h, false, true, p->rho0, p->c0, p->gamma, cap, p->block_sph,
                              p->lanes_sph, nbr_cap(c, p), p->nbr_format);
     }
     cudaGraph_t body_done = nullptr;
@@ -1050,7 +1050,7 @@ int sphdem_profile_step(sphdem_ctx_t* c, const sphdem_params_t* p, int step, int
         if (coupled && (rc = build_grid(&c->grid_dem, c->dem.pos, c->ctl, st))) break;
         mark();
         if (shep && (rc = gather_wall_rho(c, st))) break;
-        if ((rc = run_density(c, p->support, p->h, shep, true, true, p->rho0, p->c0, p->gamma, st, p->block_sph,
+        if ((rc = run_density(c, p->support, p->h, shep, true, p->rho0, p->c0, p->gamma, st, p->block_sph,
                               p->lanes_sph, nbr_cap(c, p), p->nbr_format)))
             break;
         mark();
@@ -1138,11 +1138,11 @@ int sphdem_release(sphdem_ctx_t* c) {
 
 int sphdem_shepard_sph(sphdem_ctx_t* c, float support, float h, sphdem_stream_t s) {
     if (!valid_ctx(c)) return SPHDEM_ERR_INVALID;
-    return run_density(c, support, h, true, false, false, 1.f, 1.f, 1.f, as_stream(s));
+    return run_density(c, support, h, true, false, 1.f, 1.f, 1.f, as_stream(s));
 }
 int sphdem_density_sph(sphdem_ctx_t* c, float support, float h, sphdem_stream_t s) {
     if (!valid_ctx(c)) return SPHDEM_ERR_INVALID;
-    return run_density(c, support, h, false, true, false, 1.f, 1.f, 1.f, as_stream(s));
+    return run_density(c, support, h, false, false, 1.f, 1.f, 1.f, as_stream(s));
 }
 int sphdem_density_bnd(sphdem_ctx_t* c, float support, float h, sphdem_stream_t s) {
     if (!valid_ctx(c)) return SPHDEM_ERR_INVALID;

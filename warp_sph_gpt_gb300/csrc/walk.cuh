@@ -75,12 +75,6 @@ __device__ __forceinline__ float ordered_fma(float acc, float a, float b) {
         acc = fmaf(L == 1 ? a : __shfl_sync(0xffffffffu, a, s, L), L == 1 ? b : __shfl_sync(0xffffffffu, b, s, L), acc);
     return acc;
 }
-template <int L>
-__device__ __forceinline__ float ordered_add(float acc, float a) {
-#pragma unroll
-    for (int s = 0; s < L; ++s) acc += L == 1 ? a : __shfl_sync(0xffffffffu, a, s, L);
-    return acc;
-}
 
 // Calls body(ok, j, q, r), by all 32 lanes of the warp together, until every
 // slot j of g with d2 < s2 has been given to one of the L lanes of its subject
