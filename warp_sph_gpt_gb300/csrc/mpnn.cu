@@ -1061,7 +1061,11 @@ __device__ __forceinline__ void store_colsum(float4 s, int cols, float* __restri
         const float4 o = red[k][t];
         s = make_float4(s.x + o.x, s.y + o.y, s.z + o.z, s.w + o.w);
     }
-    reinterpret_cast<float4*>(part + (size_t)blockIdx.x * cols)[t] = s;
+    float* to = part + (size_t)blockIdx.x * cols + 4 * t;  // the caller's scratch: any alignment
+    to[0] = s.x;
+    to[1] = s.y;
+    to[2] = s.z;
+    to[3] = s.w;
 }
 
 // out = d * silu'(z) as BF16 and its column sums (one partial row per CTA), for
