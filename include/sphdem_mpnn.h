@@ -102,7 +102,8 @@ typedef struct sphdem_mpnn_net {
     int32_t* active_list;     /* [1 + n_nodes - n_recv]: count, then nodes    */
 } sphdem_mpnn_net_t;
 
-/* Backward workspace (the [.., 128] buffers 16-byte aligned, as those above). */
+/* Backward workspace.  x, the [.., 128] buffers, bf_b and net.out are 16-byte
+ * aligned (SPHDEM_ERR_INVALID otherwise); d_out, partial and grad lie at any float. */
 typedef struct sphdem_mpnn_grad {
     const float* d_out;       /* [n_recv,16] dL/d out                         */
     float* g2;                /* [n_recv,128]                                 */

@@ -26,6 +26,7 @@
 #include <stdio.h>
 
 #include <map>
+#include <initializer_list>
 #include <mutex>
 #include <utility>
 
@@ -1448,6 +1449,14 @@ int edges(const EdgeArgs& a, int grid, cudaStream_t st) {
     return launch_status("mpnn edges");
 }
 
+// The rows of these buffers are moved 16 bytes at a time.
+bool aligned16(std::initializer_list<const void*> buffers) {
+    uintptr_t bits = 0;
+    for (const void* p : buffers) bits |= (uintptr_t)p;
+    if (bits & 15u) set_error_msg("mpnn: row buffers must be 16-byte aligned");
+    return (bits & 15u) == 0;
+}
+
 bool net_ok(const sphdem_mpnn_net_t* n) {
     return n && n->n_nodes >= n->n_recv && n->n_recv >= 0 && n->edge_capacity > 0 && n->node_pos4 &&
            n->node_vel4 && n->x && n->offset && n->sender && n->receiver && n->theta && n->packed && n->h0 &&
@@ -1548,6 +1557,8 @@ extern "C" int sphdem_mpnn_forward(const sphdem_mpnn_net_t* n, int store_pre, sp
         set_error_msg("mpnn_forward: invalid network state");
         return SPHDEM_ERR_INVALID;
     }
+    if (!aligned16({n->x, n->h0, n->agg, n->h1, n->h2, n->h3, n->out}) || (store_pre && !aligned16({n->z0, n->z2})))
+        return SPHDEM_ERR_INVALID;
     cudaStream_t st = as_stream(stream);
     const int nn = n->n_nodes, nr = n->n_recv;
     // node layers on the receivers and the other nodes that send (no other
@@ -1594,6 +1605,8 @@ extern "C" int sphdem_mpnn_backward(const sphdem_mpnn_net_t* n, const sphdem_mpn
         set_error_msg("mpnn_backward: invalid arguments");
         return SPHDEM_ERR_INVALID;
     }
+    if (!aligned16({n->x, n->h0, n->h1, n->h2, n->h3, n->z0, n->z2, g->g2, g->d_h2, g->d_h1, g->d_h0, g->bf_a, g->bf_b}))
+        return SPHDEM_ERR_INVALID;
     cudaStream_t st = as_stream(stream);
     const int nn = n->n_nodes, nr = n->n_recv;
     // the node rows of the forward pass
