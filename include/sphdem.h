@@ -55,7 +55,8 @@ extern "C" {
 #define SPHDEM_FLAG_ROW_OVERFLOW      0x8  /* one contact row exceeded the per-row
                                               sort buffer (rows still complete)     */
 #define SPHDEM_FLAG_TIMEOUT          0x10  /* a bounded wait on a shared-memory copy
-                                              gave up; that kernel's results are void */
+                                              gave up, after about 4 s; that kernel's
+                                              results are void */
 
 /* Opaque CUDA stream handle (cudaStream_t); 0 is the legacy default stream. */
 typedef void* sphdem_stream_t;

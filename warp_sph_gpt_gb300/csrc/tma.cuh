@@ -45,11 +45,12 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t
         : "memory");
 }
 
-// One poll.  The hint lets the hardware keep the warp suspended for up to 2 us
-// (it is woken when the phase completes); the default suspends for a small
-// part of that, and warps polling again and again took a tenth of the issue
-// slots of the porosity kernel: 2.73 -> 2.64 ms at 800k, 0.90 -> 0.86 at 100k
-// with submerged spheres.
+// One poll.  With a suspend-time hint of 2 us warps that wait beside working ones
+// take fewer issue slots: steps of 100k particles with spheres in the water 1,147
+// -> 1,109 us, above it 1,214 -> 1,185, of 792k 3,557 -> 3,465 (the porosity pass;
+// the surrogate's kernels are as fast without).  How long a wait lasts that nothing
+// ends does not depend on it: such a poll returns after 3.8 us with the hint and
+// without, so the limit of 2^20 polls that the kernels pass is 4 s.
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
