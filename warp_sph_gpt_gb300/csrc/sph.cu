@@ -42,8 +42,13 @@ namespace {
 extern __shared__ __align__(16) unsigned char sph_smem[];
 
 // kern_w(k, fast_sqrt(d2)) of a finite d2, same bits: the guard of the root at
-// 0 and the end of the support are a maximum each.
+// 0 and the end of the support are a maximum each.  Not for a warp per subject:
+// with it and Near2 that loop takes 40 registers instead of 31 and an SM holds
+// fewer warps (density of 33k particles 51 us against 43, of 387k walls 171
+// against 144).
+template <int LANES>
 __device__ __forceinline__ float member_w(const Kern& k, float d2) {
+    if (LANES == 32) return kern_w(k, fast_sqrt(d2));
     const float q = (d2 * rsqrtf(fmaxf(d2, 1.0e-37f))) * k.inv_h;
     const float u = fmaxf(1.0f - 0.5f * q, 0.0f);
     const float u2 = u * u;
@@ -117,7 +122,11 @@ __device__ __forceinline__ void visit_members(const Geo& g, const float4* __rest
         });
     } else if constexpr (LANES == 32) {
         warp_ranges_ball(g, p.x, p.y, p.z, rq, inst, [&](int s, int e) {
-            for (int j = s + lane; j < e; j += 32) one(j);
+            for (int j = s + lane; j < e; j += 32) {
+                const float4 q = posm[j];
+                const D2 r = d2_exact(p.x, p.y, p.z, q.x, q.y, q.z);
+                if (r.d2 < s2) body(true, j, q, r.d2);
+            }
         });
     } else {
         WarpWalk<LANES>* walks = reinterpret_cast<WarpWalk<LANES>*>(sph_smem);
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
         int32_t* rows = a.nbr;
         const int wf = walk_record(a.gs, a.f_posm, p, a.rq, inst, a.s2, rows, n, k, a.cap,
                                    [&](int j, const float4& q, float d2) {
-                                       const float w = member_w(a.kern, d2);
+                                       const float w = member_w<LANES>(a.kern, d2);
                                        if (RHO) rho_sum += q.w * w;
                                        if (FLT) flt_sum += a.f_vprev[j] * w;
                                    });
@@ -216,7 +225,7 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
         if (a.gb.ncl > 0)
             wb = walk_record(a.gb, a.b_posm, p, a.rq, inst, a.s2, rows + (size_t)a.cap * n, n, k, a.cap,
                              [&](int j, const float4& q, float d2) {
-                                 const float w = member_w(a.kern, d2);
+                                 const float w = member_w<LANES>(a.kern, d2);
                                  if (RHO) rho_sum += q.w * w;
                                  if (FLT) flt_sum += a.b_vprev[j] * w;
                              });
@@ -232,7 +241,7 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
             visit_members<LANES, kBatch>(g, posm, mine, p, a.rq, a.s2, inst, lane, [&](bool ok, int j,
                                                                                       const float4& q, float d2) {
                 if constexpr (LANES == 1 || LANES == 32) {
-                    const float w = member_w(a.kern, d2);
+                    const float w = member_w<LANES>(a.kern, d2);
                     if (RHO) rho_sum += q.w * w;
                     if (FLT) flt_sum += vprev[j] * w;
                     if (list) {
@@ -240,7 +249,7 @@ __global__ void __launch_bounds__(256) k_density(DensArgs a) {
                         ++found;
                     }
                 } else {
-                    const float w = ok ? member_w(a.kern, d2) : 0.0f;
+                    const float w = ok ? member_w<LANES>(a.kern, d2) : 0.0f;
                     if (list) {
                         const unsigned of = (__ballot_sync(0xffffffffu, ok) >> shift) & ((1u << (LANES & 31)) - 1u);
                         const int row = found + __popc(of & ((1u << lane) - 1u));
@@ -320,10 +329,10 @@ __global__ void __launch_bounds__(256) k_density_wall(WallArgs a) {
         visit_members<LANES>(a.gs, a.f_posm, mine, p, a.rq, a.s2, inst, lane,
                              [&](bool ok, int j, const float4& q, float d2) {
                                  if constexpr (LANES == 1 || LANES == 32)
-                                     rho_sum += q.w * member_w(a.kern, d2);
+                                     rho_sum += q.w * member_w<LANES>(a.kern, d2);
                                  else
                                      rho_sum = ordered_fma<LANES>(rho_sum, ok ? q.w : 0.0f,
-                                                                  ok ? member_w(a.kern, d2) : 0.0f);
+                                                                  ok ? member_w<LANES>(a.kern, d2) : 0.0f);
                              });
     rho_sum = lanes_sum<LANES>(rho_sum);
     if (lane != 0 || !mine) return;
